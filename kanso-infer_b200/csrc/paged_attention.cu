@@ -25,6 +25,7 @@
 
 #include "glue.cuh"
 #include "kv_pool.h"
+#include "paged_prefill.h"
 
 namespace kanso {
 
@@ -887,10 +888,12 @@ int32_t kanso_cuda_paged_attention(kanso_cuda_ctx* ctx, const kanso_cuda_kv* kv,
                                 max_ctx, nullptr);
 }
 
-// Chunked-prefill attention: every query token of every sequence is one grid row whose context
-// is the prefix up to and including itself; the rows of a sequence share its block-table row.
-// The arithmetic per row is exactly the decode attention's (the reference adds -1e9 to the
-// masked scores, src/model.rs:1027-1043, which leaves exp() == 0 for them).
+// Chunked-prefill attention: tiles of query rows (paged_prefill.cu), or where a call is outside that
+// kernel's range (head_dim other than 64 and 128) or brings hardly more than one token per
+// sequence: every query token of every sequence is one grid row whose context is the prefix up to and
+// including itself; the rows of a sequence share its block-table row. The arithmetic per row is
+// then exactly the decode attention's (the reference adds -1e9 to the masked scores,
+// src/model.rs:1027-1043, which leaves exp() == 0 for them).
 int32_t kanso_cuda_paged_attention_prefill(kanso_cuda_ctx* ctx, const kanso_cuda_kv* kv,
                                            uint32_t layer, const float* q,
                                            const uint32_t* block_tables,
@@ -921,16 +924,13 @@ int32_t kanso_cuda_paged_attention_prefill(kanso_cuda_ctx* ctx, const kanso_cuda
                 "paged_attention_prefill cannot be captured in a CUDA graph (its row arrays are "
                 "per-call host data)");
   const uint64_t cap = (uint64_t)params->max_num_blocks_per_seq * params->block_size;
-  std::vector<uint32_t> rows;  // [row_seq | row_ctx]
   uint64_t T = 0;
   for (uint32_t s = 0; s < params->num_seqs; ++s) T += host_query_lens[s];
   if (T == 0) return fail(ctx, KANSO_ERR_SHAPE, "paged_attention_prefill: no query tokens");
   if (T > (1u << 20))
     return fail(ctx, KANSO_ERR_UNSUPPORTED, "paged_attention_prefill: %llu query tokens",
                 (unsigned long long)T);
-  rows.resize(2 * T);
   uint32_t max_ctx = 0;
-  uint64_t t = 0;
   for (uint32_t s = 0; s < params->num_seqs; ++s) {
     const uint32_t ql = host_query_lens[s], cl = host_context_lens[s];
     // forward_batch_rows' checks (src/model.rs:1434-1455): the context includes the chunk
@@ -938,29 +938,32 @@ int32_t kanso_cuda_paged_attention_prefill(kanso_cuda_ctx* ctx, const kanso_cuda
       return fail(ctx, KANSO_ERR_SHAPE,
                   "paged_attention_prefill: sequence %u: context %u, %u query tokens, table "
                   "capacity %llu", s, cl, ql, (unsigned long long)cap);
-    for (uint32_t i = 0; i < ql; ++i, ++t) {
-      rows[t] = s;
-      rows[T + t] = cl - ql + i + 1;  // query i sits at position cl - ql + i
-    }
     if (cl > max_ctx) max_ctx = cl;
   }
-  // one grid row per query token; the row arrays are stream-ordered temporaries
   kanso_paged_attention_params pr = *params;
   pr.num_seqs = (uint32_t)T;
   if ((st = validate_params(&pr, msg, sizeof msg))) return fail(ctx, st, "%s", msg);
-  uint32_t* drows = nullptr;
-  KANSO_CUDA_TRY(ctx, cudaMallocAsync((void**)&drows, 2 * T * sizeof(uint32_t), ctx->stream),
-                 "paged_attention_prefill: row arrays");
-  cudaError_t ce = cudaMemcpyAsync(drows, rows.data(), 2 * T * sizeof(uint32_t),
-                                   cudaMemcpyHostToDevice, ctx->stream);
-  if (ce == cudaSuccess) {
-    st = launch_paged_attention_rows(ctx, kv, layer, q, block_tables, drows + T, out, &pr, max_ctx,
+  bool handled = false;
+  st = launch_paged_prefill(ctx, kv, layer, q, block_tables, host_context_lens, host_query_lens,
+                            out, params, &handled);
+  if (st || handled) return st;
+  // one grid row per query token: [row_seq | row_ctx]
+  std::vector<uint32_t> rows(2 * T);
+  uint64_t t = 0;
+  for (uint32_t s = 0; s < params->num_seqs; ++s)
+    for (uint32_t i = 0; i < host_query_lens[s]; ++i, ++t) {
+      rows[t] = s;
+      // query i sits at position context - query_len + i
+      rows[T + t] = host_context_lens[s] - host_query_lens[s] + i + 1;
+    }
+  if ((st = ctx_stage_dev(ctx, 2 * T * sizeof(uint32_t)))) return st;
+  uint32_t* drows = (uint32_t*)ctx->stage_dev;
+  KANSO_CUDA_TRY(ctx,
+                 cudaMemcpyAsync(drows, rows.data(), 2 * T * sizeof(uint32_t),
+                                 cudaMemcpyHostToDevice, ctx->stream),
+                 "paged_attention_prefill: row arrays to device");
+  return launch_paged_attention_rows(ctx, kv, layer, q, block_tables, drows + T, out, &pr, max_ctx,
                                      nullptr, drows);
-  } else {
-    st = cuda_fail(ctx, ce, "paged_attention_prefill: row arrays to device");
-  }
-  cudaFreeAsync(drows, ctx->stream);
-  return st;
 }
 
 }  // extern "C"
