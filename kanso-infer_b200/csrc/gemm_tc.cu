@@ -7,7 +7,7 @@
 // This is the three-product form used by the decode step's chain of matmuls (more than 8
 // sequences) and by shapes whose rows do not start on 16-byte boundaries; single matmuls of 9..512
 // rows with aligned rows take the TMA-staged kernel in gemm_tma.cu, KANSO_ACT_Q8 batches the
-// kind::i8 kernel in gemm_i8.cu.
+// weight-streaming kernel in gemm_few.cu.
 //
 // Mapping. The weight matrix is the 128-row operand of the MMA (A, K-major) and the
 // activations are the narrow operand (B, K-major, 16..128 rows), so one CTA owns 128 weight

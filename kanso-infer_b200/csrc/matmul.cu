@@ -18,11 +18,33 @@ int32_t q8_mma_matmul(kanso_cuda_ctx* ctx, int nseg, const void* const* w, float
 
 int32_t tma_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const float* x, float* y,
                    int64_t M, int64_t N, int64_t K, bool* handled);
-int32_t i8_matmul(kanso_cuda_ctx* ctx, const void* w, const float* x, float* y, int64_t M,
-                  int64_t N, int64_t K, bool* handled);
+int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const float* x, float* y,
+                   int64_t M, int64_t N, int64_t K, int32_t act_mode, bool* handled);
 
 int32_t matmul_dispatch(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const float* x,
                         float* y, int64_t M, int64_t N, int64_t K, int32_t act_mode) {
+  // 9..64 activation rows (Q8_0: from two rows on), and any number above 8 with Q8 activations: the
+  // weight-streaming kernel, in passes of at most 64 (128) rows. Against the kernels below, which
+  // keep what it does not take, us per product with weights from memory (14336 x 4096): Q8_0 at
+  // 2 / 24 / 64 rows 22 / 29 / 50 against 42 / 46 / 50; Q4_K at 16 / 24 / 64 rows 26 / 30 / 50
+  // against 46 / 48 / 54. Fewer Q4_K rows keep the int8 GEMV's finer activations. Q8 activations
+  // at 32 / 64 rows: 39 / 64 against the 128 / 129 of a tcgen05 kind::i8 form that drained an
+  // accumulator per block.
+  const bool few = act_mode == KANSO_ACT_Q8 ? M > 8 && dtype == KANSO_DTYPE_Q8_0
+                                            : M <= 64 && M >= (dtype == KANSO_DTYPE_Q8_0 ? 2 : 9);
+  if (few && w && x && y) {
+    bool all = true;
+    for (int64_t m0 = 0; m0 < M && all;) {
+      int64_t mc = M - m0 < 128 ? M - m0 : 128;
+      if (M - m0 - mc > 0 && M - m0 - mc < 9) mc -= 16;  // no short tail
+      bool handled = false;
+      int32_t st = few_matmul(ctx, dtype, w, x + m0 * K, y + m0 * N, mc, N, K, act_mode, &handled);
+      if (st != KANSO_OK) return st;
+      if (!handled) all = false;
+      m0 += mc;
+    }
+    if (all) return KANSO_OK;
+  }
   // More than 8 activation rows on a matrix whose rows start on 16-byte boundaries: the
   // TMA-staged tcgen05 GEMM, up to 512 rows per pass over the weights. Q8_0 takes it from two
   // rows on: measured on 14336 x 4096 / 4096 x 4096 / 4096 x 14336 it needs 31.8 / 11.9 / 30.0 us
@@ -54,22 +76,6 @@ int32_t matmul_dispatch(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const
                              K, &handled);
       if (st != KANSO_OK) return st;
       if (!handled) all = false;
-    }
-    if (all) return KANSO_OK;
-  }
-  // Q8_0 weights with Q8 activations and more than 8 rows: int8 tensor-core GEMM with exact
-  // int32 block sums, 128 rows per pass over the weights
-  if (M > 8 && act_mode == KANSO_ACT_Q8 && dtype == KANSO_DTYPE_Q8_0 && N > 0 && K > 0 && w && x &&
-      y) {
-    bool all = true;
-    for (int64_t m0 = 0; m0 < M && all;) {
-      int64_t mc = M - m0 < 128 ? M - m0 : 128;
-      if (M - m0 - mc > 0 && M - m0 - mc < 9) mc -= 16;  // a short tail rides with this chunk
-      bool handled = false;
-      int32_t st = i8_matmul(ctx, w, x + m0 * K, y + m0 * N, mc, N, K, &handled);
-      if (st != KANSO_OK) return st;
-      if (!handled) all = false;
-      m0 += mc;
     }
     if (all) return KANSO_OK;
   }
