@@ -27,7 +27,7 @@
 
 #include "kv_pool.h"
 #include "paged_prefill.h"
-#include "warp_mma.cuh"
+#include "pool_mma.cuh"
 
 namespace kanso {
 
@@ -59,50 +59,6 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool in) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n)
                : "memory");
 }
-__device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                       uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                        uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-// x = hi + lo, two values at a time
-__device__ __forceinline__ void split_f16(float x0, float x1, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(x0, x1);
-  const float2 f = __half22float2(h);
-  hi = h2_bits(h);
-  lo = h2_bits(__floats2half2_rn(x0 - f.x, x1 - f.y));
-}
-// Four bytes of the pool as two f16 pairs, exactly.
-template <bool FP8>
-__device__ __forceinline__ uint2 bytes_to_f16(uint32_t w) {
-  uint2 r;
-  if (FP8) {
-    __half2_raw a = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w & 0xFFFFu), __NV_E4M3);
-    __half2_raw b = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3);
-    r.x = h2_bits(__half2(a));
-    r.y = h2_bits(__half2(b));
-  } else {
-    // value + 128 in the low byte of 1024's f16 pattern, minus 1152
-    w ^= 0x80808080u;
-    const __half2 off = __float2half2_rn(1152.f);
-    uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
-    r.x = h2_bits(__hsub2(*reinterpret_cast<__half2*>(&a), off));
-    r.y = h2_bits(__hsub2(*reinterpret_cast<__half2*>(&b), off));
-  }
-  return r;
-}
-
 // Shared memory: raw K and V rows [2][64][HD] each (16-byte chunks swizzled for the matrix loads of
 // K), V as f16 [64][HD] (and K, fp8), the raw scales [2][2][64], the derived ones [3][64].
 template <int HD, bool FP8>
@@ -256,12 +212,8 @@ __global__ void __launch_bounds__(PP_WARPS * 32, HD == 64 ? 3 : 2)
         }
       top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
       top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
-      // a power of two that brings the row under one, from the exponent's bits (a row beyond the
-      // normal numbers keeps its values)
-      const int e = (int)(__float_as_uint(top) >> 23);
-      const bool ok = e >= 2 && e <= 252;
-      const float down = ok ? __uint_as_float((uint32_t)(253 - e) << 23) : 1.f;
-      cr[h] = ok ? __uint_as_float((uint32_t)(e + 1) << 23) : 1.f;
+      float down;
+      pow2_scale(top, cr[h], down);
 #pragma unroll
       for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
@@ -307,7 +259,7 @@ __global__ void __launch_bounds__(PP_WARPS * 32, HD == 64 ? 3 : 2)
       const float* sc = reinterpret_cast<const float*>(smem + S::sc) + st * 2 * PP_TOK;
       float* d = reinterpret_cast<float*>(smem + S::der);
       const float vs = fmaxf(sc[PP_TOK + tid], 1.17549435e-38f);
-      d[tid] = sc[tid] * (a.scale * 1.4426950408889634f);
+      d[tid] = sc[tid] * a.scale;
       d[PP_TOK + tid] = __log2f(vs);
       d[2 * PP_TOK + tid] = 1.0f / vs;
     }
@@ -370,7 +322,8 @@ __global__ void __launch_bounds__(PP_WARPS * 32, HD == 64 ? 3 : 2)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float x = FP8 ? t_[j][e] : (float)sc_i[j][e];
-        t_[j][e] = fmaf(x * cr[e >> 1], (e & 1) ? ks2.y : ks2.x, (e & 1) ? lv2.y : lv2.x);
+        t_[j][e] = log2_score(x * cr[e >> 1] * ((e & 1) ? ks2.y : ks2.x),
+                              (e & 1) ? lv2.y : lv2.x);
       }
     }
     if ((int)(i * PP_TOK + PP_TOK - 1) > wmin) {  // some row of the warp does not see all of it
