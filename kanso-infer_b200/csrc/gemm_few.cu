@@ -9,8 +9,8 @@
 // hundred rows. mma.sync reaches 1024 (f16) and 2048 (int8) multiply-adds per clock and SM here,
 // which is enough up to about 64 rows.
 //
-//   * A unit is 128 weight rows x 256 k: one tensor-map copy of 128 x 272 (Q8_0) or 128 x 144
-//     (Q4_K) bytes, whole blocks, in rows whose stride is 16 bytes past a multiple of 128, so that
+//   * A unit is 128 weight rows (int8 form: 112) x 256 k: one tensor-map copy of 272 (Q8_0) or 144
+//     (Q4_K) bytes a row, whole blocks, in rows whose stride is 16 bytes past a multiple of 128, so that
 //     8 rows x 4 lanes of 4-byte reads meet 32 different banks without a swizzle.
 //   * Units are numbered tile by tile and dealt out in equal contiguous runs; the runs ignore tile
 //     borders, so there is no last wave. A run that ends inside a tile adds its sums to y with
@@ -38,10 +38,16 @@ namespace kanso {
 
 enum FewForm { FEW_Q8_F16, FEW_Q4_F16, FEW_Q8_INT8 };
 
-constexpr int FEW_TILE = 128;  // weight rows of a unit
 constexpr int FEW_K = 256;     // k of a unit
 constexpr int FEW_MAX_STAGES = 6;
 
+// Weight rows of a unit. INT8: whole rows of K per CTA, bound by the arithmetic of the SMs that have
+// one: 112 rows give a matrix of 14336 rows to 128 SMs where 128 rows give it to 112 (128 activation
+// rows 106 -> 100 us, 4096 x 14336 99 -> 95 us).
+template <int FORM>
+__host__ __device__ constexpr int few_tile() {
+  return FORM == FEW_Q8_INT8 ? 112 : 128;
+}
 template <int FORM>
 __host__ __device__ constexpr int few_row_bytes() {  // of one weight row in a unit
   return FORM == FEW_Q4_F16 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES;
@@ -301,12 +307,10 @@ __device__ __forceinline__ void few_unit_q4_f16(float (&acc)[2][NT][4], const ui
   }
 }
 
-// INT8 form: one block of the warp's RT x 16 rows against `tiles` (at most NT) groups of 8
-// activation rows.
+// INT8 form: one block of the warp's RT x 16 rows against NT groups of 8 activation rows.
 template <int RT, int NT, bool ODD>
 __device__ __forceinline__ void few_int8_block(float (&acc)[RT][NT][4], const uint8_t* w,
-                                               const uint8_t* x, const uint8_t* dx, int t,
-                                               int tiles) {
+                                               const uint8_t* x, const uint8_t* dx, int t) {
   uint32_t a[RT][4];
   uint64_t dw[RT][2];
 #pragma unroll
@@ -319,7 +323,6 @@ __device__ __forceinline__ void few_int8_block(float (&acc)[RT][NT][4], const ui
   }
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
-    if (n >= tiles) break;
     const uint2 b = lds<uint2>(x + n * 8 * FEW_K);
     const uint2 d2 = lds<uint2>(dx + n * 32);
     const uint64_t dxp = f32x2(d2.x, d2.y);
@@ -343,16 +346,15 @@ __device__ __forceinline__ void few_int8_block(float (&acc)[RT][NT][4], const ui
 template <int RT, int NT>
 __device__ __forceinline__ void few_unit_int8(float (&acc)[RT][NT][4], const uint8_t* w,
                                               const uint8_t* x, const uint8_t* dx, int Mp, int g,
-                                              int t, int tiles) {
+                                              int t) {
   w += g * few_row_bytes<FEW_Q8_INT8>();
   x += g * FEW_K + t * 8;
   dx += t * 8;
 #pragma unroll
   for (int b = 0; b < 8; b += 2) {
-    few_int8_block<RT, NT, false>(acc, w + b * Q8_BYTES, x + (b ^ (g & 3)) * 32, dx + b * Mp * 4, t,
-                                  tiles);
+    few_int8_block<RT, NT, false>(acc, w + b * Q8_BYTES, x + (b ^ (g & 3)) * 32, dx + b * Mp * 4, t);
     few_int8_block<RT, NT, true>(acc, w + (b + 1) * Q8_BYTES, x + ((b + 1) ^ (g & 3)) * 32,
-                                 dx + (b + 1) * Mp * 4, t, tiles);
+                                 dx + (b + 1) * Mp * 4, t);
   }
 }
 
@@ -361,11 +363,11 @@ __device__ __forceinline__ void few_unit_int8(float (&acc)[RT][NT][4], const uin
 // of NT x 8). No wait is unbounded: after one that ran out a warp skips its work but still takes
 // part in the barriers of its row group.
 template <int FORM, int RT, int NT, int OTHER, int CTAS>
-__global__ void __launch_bounds__(FEW_TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
+__global__ void __launch_bounds__(few_tile<FORM>() / (16 * RT) * OTHER * 32 + 32, CTAS)
     gemm_few_kernel(const __grid_constant__ CUtensorMap tmap, const FewArgs a) {
-  constexpr int WR = FEW_TILE / (16 * RT), WARPS = WR * OTHER;
+  constexpr int WR = few_tile<FORM>() / (16 * RT), WARPS = WR * OTHER;
   constexpr int Mp = NT * 8 * (FORM == FEW_Q8_INT8 ? OTHER : 1);
-  constexpr uint32_t W_BYTES = FEW_TILE * few_row_bytes<FORM>();
+  constexpr uint32_t W_BYTES = few_tile<FORM>() * few_row_bytes<FORM>();
   constexpr uint32_t X_BYTES = Mp * few_x_bytes<FORM>();
   constexpr uint32_t STAGE = W_BYTES + X_BYTES;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -391,7 +393,7 @@ __global__ void __launch_bounds__(FEW_TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
       auto weights = [&](int u, int slot) {
         mbar_arrive_expect_tx(&full[slot], STAGE);
         tma_load_2d(smem + slot * STAGE, &tmap, u % a.chunks * (few_row_bytes<FORM>() / 4),
-                    u / a.chunks * FEW_TILE, &full[slot]);
+                    u / a.chunks * few_tile<FORM>(), &full[slot]);
       };
       auto rows = [&](int u, int slot) {
         bulk_g2s(smem + slot * STAGE + W_BYTES, a.xp + (int64_t)(u % a.chunks) * X_BYTES, X_BYTES,
@@ -435,8 +437,7 @@ __global__ void __launch_bounds__(FEW_TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
         few_unit_q4_f16<NT>(acc, w, x, other, g, t);
       else
         few_unit_int8<RT, NT>(acc, w, x + other * NT * 8 * FEW_K,
-                              x + Mp * FEW_K + other * NT * 32, Mp, g, t,
-                              (a.M + 7) / 8 - other * NT);
+                              x + Mp * FEW_K + other * NT * 32, Mp, g, t);
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[slot]);
     }
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(FEW_TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
         asm volatile("bar.sync %0, %1;" ::"r"(1 + wr), "n"(OTHER * 32) : "memory");
       }
     }
-    const int64_t n0 = (int64_t)(u / a.chunks) * FEW_TILE + wr * (16 * RT) + g;
+    const int64_t n0 = (int64_t)(u / a.chunks) * few_tile<FORM>() + wr * (16 * RT) + g;
     const int m0 = (FORM == FEW_Q8_INT8 ? other * NT * 8 : 0) + 2 * t;
     if (ok && (FORM == FEW_Q8_INT8 || other == 0))
 #pragma unroll
@@ -499,9 +500,9 @@ __global__ void __launch_bounds__(FEW_TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
 
 template <int FORM, int RT, int NT, int OTHER, int CTAS>
 static int32_t few_launch(kanso_cuda_ctx* ctx, const CUtensorMap& map, FewArgs a, int grid) {
-  constexpr int WR = FEW_TILE / (16 * RT);
+  constexpr int WR = few_tile<FORM>() / (16 * RT);
   constexpr int Mp = NT * 8 * (FORM == FEW_Q8_INT8 ? OTHER : 1);
-  constexpr size_t stage = FEW_TILE * few_row_bytes<FORM>() + Mp * few_x_bytes<FORM>();
+  constexpr size_t stage = few_tile<FORM>() * few_row_bytes<FORM>() + Mp * few_x_bytes<FORM>();
   constexpr size_t slab =
       FORM == FEW_Q8_INT8 ? 0 : (OTHER - 1) * WR * RT * (NT < 2 ? NT : 2) * 4 * 32 * 4;
   // CTAS blocks share an SM's memory, of which each needs 1 KB besides and its static part
@@ -548,7 +549,8 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   if (M < 1 || M > (int8 ? 128 : 64) || N < 1 || K < FEW_K || K % FEW_K != 0 || !w || !x || !y)
     return KANSO_OK;
   const int64_t row_bytes = K / FEW_K * (q4 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES);
-  const int64_t chunks = K / FEW_K, tiles = (N + FEW_TILE - 1) / FEW_TILE;
+  const int tile = int8 ? few_tile<FEW_Q8_INT8>() : few_tile<FEW_Q8_F16>();
+  const int64_t chunks = K / FEW_K, tiles = (N + tile - 1) / tile;
   if (!aligned16(w) || row_bytes > (1 << 28) || tiles * chunks > (1 << 30) || N > (1 << 30))
     return KANSO_OK;
   TmEncodeFn encode = tm_encoder();
@@ -556,7 +558,8 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   CUtensorMap map;
   const cuuint64_t gdim[2] = {(cuuint64_t)row_bytes / 4, (cuuint64_t)N};
   const cuuint64_t gstride[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)(q4 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES) / 4, FEW_TILE};
+  const cuuint32_t box[2] = {(cuuint32_t)(q4 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES) / 4,
+                             (cuuint32_t)tile};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(w), gdim,
                              gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -581,7 +584,8 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
       split *= 2;
     grid = (int)tiles * split;
     a.add = split > 1;
-    nt = M <= 32 ? 4 : M <= 64 ? 8 : 16;
+    // groups of rows for 1, 2 or 4 warps of a row group (a test per group cost 45 % at 32 rows)
+    nt = M <= 16 ? 2 : M <= 24 ? 3 : M <= 32 ? 4 : M <= 48 ? 6 : M <= 64 ? 8 : M <= 96 ? 12 : 16;
   } else {
     a.add = true;
     if (nt > 4) nt = nt <= 6 ? 6 : 8;
@@ -611,9 +615,15 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   if (!int8)
     return q4 ? few_launch_f16<FEW_Q4_F16>(ctx, nt, map, a)
               : few_launch_f16<FEW_Q8_F16>(ctx, nt, map, a);
-  if (nt == 4) return few_launch<FEW_Q8_INT8, 1, 4, 1, 1>(ctx, map, a, grid);
-  if (nt == 8) return few_launch<FEW_Q8_INT8, 1, 4, 2, 1>(ctx, map, a, grid);
-  return few_launch<FEW_Q8_INT8, 2, 4, 4, 1>(ctx, map, a, grid);
+  switch (nt) {
+    case 2: return few_launch<FEW_Q8_INT8, 1, 2, 1, 1>(ctx, map, a, grid);
+    case 3: return few_launch<FEW_Q8_INT8, 1, 3, 1, 1>(ctx, map, a, grid);
+    case 4: return few_launch<FEW_Q8_INT8, 1, 4, 1, 1>(ctx, map, a, grid);
+    case 6: return few_launch<FEW_Q8_INT8, 1, 3, 2, 1>(ctx, map, a, grid);
+    case 8: return few_launch<FEW_Q8_INT8, 1, 4, 2, 1>(ctx, map, a, grid);
+    case 12: return few_launch<FEW_Q8_INT8, 1, 3, 4, 1>(ctx, map, a, grid);
+    default: return few_launch<FEW_Q8_INT8, 1, 4, 4, 1>(ctx, map, a, grid);
+  }
 }
 
 }  // namespace kanso

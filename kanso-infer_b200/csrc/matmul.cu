@@ -28,8 +28,8 @@ int32_t matmul_dispatch(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const
   // keep what it does not take, us per product with weights from memory (14336 x 4096): Q8_0 at
   // 2 / 24 / 64 rows 22 / 29 / 50 against 42 / 46 / 50; Q4_K at 16 / 24 / 64 rows 26 / 30 / 50
   // against 46 / 48 / 54. Fewer Q4_K rows keep the int8 GEMV's finer activations. Q8 activations
-  // at 32 / 64 rows: 39 / 64 against the 128 / 129 of a tcgen05 kind::i8 form that drained an
-  // accumulator per block.
+  // at 16 / 32 / 64 / 128 rows: 27 / 38 / 61 / 100 against the 127 / 128 / 129 / 168 of a tcgen05
+  // kind::i8 form that drained an accumulator per block.
   const bool few = act_mode == KANSO_ACT_Q8 ? M > 8 && dtype == KANSO_DTYPE_Q8_0
                                             : M <= 64 && M >= (dtype == KANSO_DTYPE_Q8_0 ? 2 : 9);
   if (few && w && x && y) {
