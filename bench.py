@@ -304,7 +304,7 @@ def gemm_legs(torch, kb, O, ctx, stream):
                     "bound": bound, "frac_of_bound": frac}
                 if dtype == kb.DTYPE_Q8_0 and rows == 14336 and M in (32, 128):
                     # the bit-exact mode: activations quantised per 32 (quantize_row_q8_0), int32
-                    # block sums on tcgen05 kind::i8
+                    # block sums
                     def step_q8():
                         for w_ in ws:
                             f(w_, x, y, M, rows, K, kb.ACT_Q8)
