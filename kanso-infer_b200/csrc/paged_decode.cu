@@ -16,7 +16,9 @@
 //     and the V words that a lane needs come from different banks.
 //   * values: A = V^T from pairs of tokens' words as f16 (exact), sums of a tile in the tensor core,
 //     across tiles in f32 registers. The V scale goes into the weights: w = 2^(s + log2 vs - max),
-//     the denominator takes w / vs.
+//     the denominator takes w / vs (pool_mma.cuh: unless scales are out of the ordinary).
+#include <type_traits>
+
 #include "paged_attention.cuh"
 #include "pool_mma.cuh"
 
@@ -92,12 +94,13 @@ __global__ void __launch_bounds__(PD_NT, HD == 64 ? 3 : 2)
     mbar_fence_init();
   }
   __syncwarp();
-  auto load = [&](uint32_t i) {  // all lanes: tile i of the warp into slot i % SLOTS
+  // all lanes: tile i of the warp into the slot of the p-th copy, p % SLOTS
+  auto load = [&](uint32_t i, uint32_t p) {
     if (i && i % 32 == 0) blocks = tile_block(i + lane);
     const uint32_t phys = __shfl_sync(0xFFFFFFFFu, blocks, i & 31);
     if (lane == 0) {
-      uint64_t* bar = &s_full[warp][i % SLOTS];
-      uint8_t* dst = ring + i % SLOTS * TB;
+      uint64_t* bar = &s_full[warp][p % SLOTS];
+      uint8_t* dst = ring + p % SLOTS * TB;
       const uint8_t* rec = a.g.pool + a.g.rec_offset(a.layer, phys, kvh);
       mbar_arrive_expect_tx(bar, TB);
       if (bs == PD_TILE) {
@@ -113,7 +116,7 @@ __global__ void __launch_bounds__(PD_NT, HD == 64 ? 3 : 2)
     }
   };
   const uint32_t ahead = min(mine, SLOTS);
-  for (uint32_t i = 0; i < ahead; ++i) load(i);
+  for (uint32_t i = 0; i < ahead; ++i) load(i, i);
 
   uint32_t new_slot = 0;
   if (fused) {
@@ -247,153 +250,207 @@ __global__ void __launch_bounds__(PD_NT, HD == 64 ? 3 : 2)
   }
 
   float m[HT], l[HT], acc[HT][2 * NV][2];
-#pragma unroll
-  for (int ht = 0; ht < HT; ++ht) {
-    m[ht] = -INFINITY;
-    l[ht] = 0.f;
-#pragma unroll
-    for (int j = 0; j < 2 * NV; ++j) acc[ht][j][0] = acc[ht][j][1] = 0.f;
-  }
+  float unit[HT];  // what acc counts in
   const uint32_t ka = (g & 1) ? 4 + ((g >> 1) ^ 1) : g >> 1;  // rows g and g + 8 of A: ka, ka + 8
-  for (uint32_t i = 0; i < mine; ++i) {
-    uint8_t* slot = ring + i % SLOTS * TB;
-    // bounded: a copy that never lands is reported, the warp carries on with what it has
-    if (!mbar_wait_bounded(&s_full[warp][i % SLOTS], (i / SLOTS) & 1u) && lane == 0)
-      atomicOr(a.status, DEV_WAIT_TIMEOUT);
-    const uint32_t first = (warp + i * PD_WARPS) * PD_TILE;  // of the partition
-    if (writer && i + 1 == mine) {
+  // All tiles in order, as the ring's next copies; false: the careful form is asked for.
+  auto walk = [&](auto careful) {
+    constexpr bool CAREFUL = decltype(careful)::value;
+    uint32_t seen = 0;
 #pragma unroll
-      for (int kv = 0; kv < 2; ++kv) {
+    for (int ht = 0; ht < HT; ++ht) {
+      m[ht] = -INFINITY;
+      l[ht] = 0.f;
+      unit[ht] = CAREFUL ? 0.f : 1.f;
 #pragma unroll
-        for (int e = 0; e < QE; ++e)
-          slot[(kv * PD_TILE + i_new - first) * HD + lane + 32 * e] =
-              (uint8_t)(new_q[kv] >> (8 * e));
-        if (lane == 0)
-          reinterpret_cast<float*>(slot + 2 * PD_TILE * HD)[kv * PD_TILE + i_new - first] =
-              new_scale[kv];
+      for (int j = 0; j < 2 * NV; ++j) acc[ht][j][0] = acc[ht][j][1] = 0.f;
+    }
+    for (uint32_t i = 0; i < mine; ++i) {
+      const uint32_t p = CAREFUL ? mine + i : i;
+      uint8_t* slot = ring + p % SLOTS * TB;
+      // bounded: a copy that never lands is reported, the warp carries on with what it has
+      if (!mbar_wait_bounded(&s_full[warp][p % SLOTS], (p / SLOTS) & 1u) && lane == 0)
+        atomicOr(a.status, DEV_WAIT_TIMEOUT);
+      const uint32_t first = (warp + i * PD_WARPS) * PD_TILE;  // of the partition
+      if (writer && i + 1 == mine) {
+#pragma unroll
+        for (int kv = 0; kv < 2; ++kv) {
+#pragma unroll
+          for (int e = 0; e < QE; ++e)
+            slot[(kv * PD_TILE + i_new - first) * HD + lane + 32 * e] =
+                (uint8_t)(new_q[kv] >> (8 * e));
+          if (lane == 0)
+            reinterpret_cast<float*>(slot + 2 * PD_TILE * HD)[kv * PD_TILE + i_new - first] =
+                new_scale[kv];
+        }
+        __syncwarp();
       }
+      const uint8_t* kr = slot;
+      const uint8_t* vr = slot + PD_TILE * HD;
+      const float* ks = reinterpret_cast<const float*>(slot + 2 * PD_TILE * HD);
+      const float* vs = ks + PD_TILE;
+      const bool in0 = first + ka < n, in1 = first + ka + 8 < n, whole = first + PD_TILE <= n;
+
+      // ---- V words of tokens t, 4 + (t ^ 1) and the same + 8, by pairs ----
+      uint32_t vw[4][NV];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t tk = ((r & 1) ? 4 + (t ^ 1) : t) + 8 * (r >> 1);
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(vr + tk * HD) + g;
+        uint32_t raw[NV];
+        if constexpr (NV == 2) {
+          raw[0] = row[8 * (t >> 1)];
+          raw[1] = row[8 * ((t >> 1) ^ 1)];
+          vw[r][0] = (t >> 1) ? raw[1] : raw[0];
+          vw[r][1] = (t >> 1) ? raw[0] : raw[1];
+        } else {
+          uint32_t one[NV];
+#pragma unroll
+          for (int j = 0; j < NV; ++j) raw[j] = row[8 * ((j + t) & 3)];
+#pragma unroll
+          for (int j = 0; j < NV; ++j) one[j] = (t & 1) ? raw[(j + 3) & 3] : raw[j];
+#pragma unroll
+          for (int j = 0; j < NV; ++j) vw[r][j] = (t & 2) ? one[(j + 2) & 3] : one[j];
+        }
+        if (!whole && first + tk >= n) {  // never written bytes: E4M3 has NaN patterns
+#pragma unroll
+          for (int j = 0; j < NV; ++j) vw[r][j] = 0;
+        }
+      }
+      float vs0 = in0 ? vs[ka] : CAREFUL ? 0.f : 1.f, vs1 = in1 ? vs[ka + 8] : CAREFUL ? 0.f : 1.f;
+      const float ks0 = ks[ka], ks1 = ks[ka + 8];
+      uint4 k0[HD / 64], k1[HD / 64];
+#pragma unroll
+      for (int c = 0; c < HD / 64; ++c) {
+        k0[c] = *reinterpret_cast<const uint4*>(kr + ka * HD + (t + 4 * c) * 16);
+        k1[c] = *reinterpret_cast<const uint4*>(kr + (ka + 8) * HD + (t + 4 * c) * 16);
+      }
+      if (CAREFUL) {
+        const uint32_t used =
+            __ballot_sync(0xFFFFFFFFu, any_value<FP8, HD / 32>(vr + lane * (HD / 2)));
+        if (!(used >> (2 * ka) & 3u)) vs0 = 0.f;
+        if (!(used >> (2 * ka + 16) & 3u)) vs1 = 0.f;
+      } else {
+        seen |= scale_bits(vs0) | scale_bits(vs1);
+      }
+      // everything of the slot is in registers: the next copy may go there
       __syncwarp();
-    }
-    const uint8_t* kr = slot;
-    const uint8_t* vr = slot + PD_TILE * HD;
-    const float* ks = reinterpret_cast<const float*>(slot + 2 * PD_TILE * HD);
-    const float* vs = ks + PD_TILE;
-    const bool in0 = first + ka < n, in1 = first + ka + 8 < n, whole = first + PD_TILE <= n;
+      if (i + SLOTS < mine) load(i + SLOTS, p + SLOTS);
 
-    // ---- V words of tokens t, 4 + (t ^ 1) and the same + 8, by pairs ----
-    uint32_t vw[4][NV];
+      // ---- scores ----
+      float x0[HT], x1[HT];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const uint32_t tk = ((r & 1) ? 4 + (t ^ 1) : t) + 8 * (r >> 1);
-      const uint32_t* row = reinterpret_cast<const uint32_t*>(vr + tk * HD) + g;
-      uint32_t raw[NV];
-      if constexpr (NV == 2) {
-        raw[0] = row[8 * (t >> 1)];
-        raw[1] = row[8 * ((t >> 1) ^ 1)];
-        vw[r][0] = (t >> 1) ? raw[1] : raw[0];
-        vw[r][1] = (t >> 1) ? raw[0] : raw[1];
-      } else {
-        uint32_t one[NV];
+      for (int ht = 0; ht < HT; ++ht) {
+        if constexpr (!FP8) {
+          int c4[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int j = 0; j < NV; ++j) raw[j] = row[8 * ((j + t) & 3)];
-#pragma unroll
-        for (int j = 0; j < NV; ++j) one[j] = (t & 1) ? raw[(j + 3) & 3] : raw[j];
-#pragma unroll
-        for (int j = 0; j < NV; ++j) vw[r][j] = (t & 2) ? one[(j + 2) & 3] : one[j];
-      }
-      if (!whole && first + tk >= n) {  // never written bytes: E4M3 has NaN patterns
-#pragma unroll
-        for (int j = 0; j < NV; ++j) vw[r][j] = 0;
-      }
-    }
-    const float vs0 = in0 ? fmaxf(vs[ka], 1.17549435e-38f) : 1.f;
-    const float vs1 = in1 ? fmaxf(vs[ka + 8], 1.17549435e-38f) : 1.f;
-    const float ks0 = ks[ka], ks1 = ks[ka + 8];
-    uint4 k0[HD / 64], k1[HD / 64];
-#pragma unroll
-    for (int c = 0; c < HD / 64; ++c) {
-      k0[c] = *reinterpret_cast<const uint4*>(kr + ka * HD + (t + 4 * c) * 16);
-      k1[c] = *reinterpret_cast<const uint4*>(kr + (ka + 8) * HD + (t + 4 * c) * 16);
-    }
-    // everything of the slot is in registers: the next copy may go there
-    __syncwarp();
-    if (i + SLOTS < mine) load(i + SLOTS);
-
-    // ---- scores ----
-    float x0[HT], x1[HT];
-#pragma unroll
-    for (int ht = 0; ht < HT; ++ht) {
-      if constexpr (!FP8) {
-        int c4[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c) {
-          mma_s8(c4, {k0[c].x, k1[c].x, k0[c].y, k1[c].y}, qb[ht][2 * c][0], qb[ht][2 * c][1]);
-          mma_s8(c4, {k0[c].z, k1[c].z, k0[c].w, k1[c].w}, qb[ht][2 * c + 1][0],
-                 qb[ht][2 * c + 1][1]);
-        }
-        x0[ht] = (float)(c4[0] * 254 + c4[1]);
-        x1[ht] = (float)(c4[2] * 254 + c4[3]);
-      } else {
-        // sums of 32 dims in the tensor core, which cuts off where an addition rounds
-        float c4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c) {
-          const uint32_t w0[4] = {k0[c].x, k0[c].y, k0[c].z, k0[c].w};
-          const uint32_t w1[4] = {k1[c].x, k1[c].y, k1[c].z, k1[c].w};
-#pragma unroll
-          for (int s = 0; s < 4; s += 2) {
-            float d4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int h = s; h < s + 2; ++h) {
-              const uint2 r0 = bytes_to_f16<true>(w0[h]), r1 = bytes_to_f16<true>(w1[h]);
-              mma_f16(d4, {r0.x, r1.x, r0.y, r1.y}, qb[ht][4 * c + h][0], qb[ht][4 * c + h][1]);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) c4[e] += d4[e];
+          for (int c = 0; c < HD / 64; ++c) {
+            mma_s8(c4, {k0[c].x, k1[c].x, k0[c].y, k1[c].y}, qb[ht][2 * c][0], qb[ht][2 * c][1]);
+            mma_s8(c4, {k0[c].z, k1[c].z, k0[c].w, k1[c].w}, qb[ht][2 * c + 1][0],
+                   qb[ht][2 * c + 1][1]);
           }
+          x0[ht] = (float)(c4[0] * 254 + c4[1]);
+          x1[ht] = (float)(c4[2] * 254 + c4[3]);
+        } else {
+          // sums of 32 dims in the tensor core, which cuts off where an addition rounds
+          float c4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c) {
+            const uint32_t w0[4] = {k0[c].x, k0[c].y, k0[c].z, k0[c].w};
+            const uint32_t w1[4] = {k1[c].x, k1[c].y, k1[c].z, k1[c].w};
+#pragma unroll
+            for (int s = 0; s < 4; s += 2) {
+              float d4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+              for (int h = s; h < s + 2; ++h) {
+                const uint2 r0 = bytes_to_f16<true>(w0[h]), r1 = bytes_to_f16<true>(w1[h]);
+                mma_f16(d4, {r0.x, r1.x, r0.y, r1.y}, qb[ht][4 * c + h][0], qb[ht][4 * c + h][1]);
+              }
+#pragma unroll
+              for (int e = 0; e < 4; ++e) c4[e] += d4[e];
+            }
+          }
+          x0[ht] = c4[0] + c4[1];
+          x1[ht] = c4[2] + c4[3];
         }
-        x0[ht] = c4[0] + c4[1];
-        x1[ht] = c4[2] + c4[3];
+      }
+      // ---- weights ----
+      const TileUnit tu = CAREFUL ? tile_unit(vs0, vs1) : TileUnit{1.f, 1.f};
+      const float lv0 = CAREFUL ? 0.f : __log2f(vs0), lv1 = CAREFUL ? 0.f : __log2f(vs1);
+      const float iv0 = CAREFUL ? vs0 * tu.up : __fdividef(1.0f, vs0);
+      const float iv1 = CAREFUL ? vs1 * tu.up : __fdividef(1.0f, vs1);
+      uint32_t pb[HT][2];
+      float f[HT];
+#pragma unroll
+      for (int ht = 0; ht < HT; ++ht) {
+        const float u0 = x0[ht] * cr[ht] * ks0, u1 = x1[ht] * cr[ht] * ks1;
+        const float s0 = !in0 ? -INFINITY : CAREFUL ? log2_units(u0) : log2_score(u0, lv0);
+        const float s1 = !in1 ? -INFINITY : CAREFUL ? log2_units(u1) : log2_score(u1, lv1);
+        float top = fmaxf(s0, s1);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+        top = fmaxf(top, m[ht]);
+        // weights up to 2^14
+        const float base = top == -INFINITY ? 0.f : CAREFUL ? top : top - 14.f;
+        f[ht] = m[ht] == -INFINITY ? 0.f : ex2_approx(m[ht] - top);
+        m[ht] = top;
+        float w0 = ex2_approx(s0 - base), w1 = ex2_approx(s1 - base);
+        if (CAREFUL) {
+          l[ht] = fmaf(l[ht], f[ht], w0 + w1);
+          w0 = fmaxf(w0 * iv0, 0.f);  // not a number: no weight, infinite scale
+          w1 = fmaxf(w1 * iv1, 0.f);
+          float largest = fmaxf(w0, w1);
+#pragma unroll
+          for (int o = 4; o < 32; o <<= 1)
+            largest = fmaxf(largest, __shfl_xor_sync(0xFFFFFFFFu, largest, o));
+          const float lift = exp2i(lift_weights(largest, tu.down, f[ht], unit[ht]));
+          w0 *= lift;
+          w1 *= lift;
+        } else {
+          l[ht] = fmaf(l[ht], f[ht], fmaf(w0, iv0, w1 * iv1));
+        }
+        pb[ht][0] = transpose_pairs(split_pair(w0));
+        pb[ht][1] = transpose_pairs(split_pair(w1));
+      }
+      // ---- values ----
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        uint32_t lo[4], hi[4];  // dims 32j + 4g + 0..3 of the first and of the second token pair
+        token_pairs<FP8>(vw[0][j], vw[1][j], lo);
+        token_pairs<FP8>(vw[2][j], vw[3][j], hi);
+#pragma unroll
+        for (int ht = 0; ht < HT; ++ht)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float d4[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_f16(d4, {lo[2 * e], lo[2 * e + 1], hi[2 * e], hi[2 * e + 1]}, pb[ht][0], pb[ht][1]);
+            float(&c)[2] = acc[ht][2 * j + e];
+            c[0] = fmaf(c[0], f[ht], d4[0] + d4[1]);
+            c[1] = fmaf(c[1], f[ht], d4[2] + d4[3]);
+          }
       }
     }
-    // ---- weights ----
-    const float lv0 = __log2f(vs0), lv1 = __log2f(vs1);
-    const float iv0 = __fdividef(1.0f, vs0), iv1 = __fdividef(1.0f, vs1);
-    uint32_t pb[HT][2];
-    float f[HT];
+    if (CAREFUL) return true;
+    bool good = !unusual_scales(seen);
 #pragma unroll
     for (int ht = 0; ht < HT; ++ht) {
-      const float s0 = in0 ? log2_score(x0[ht] * cr[ht] * ks0, lv0) : -INFINITY;
-      const float s1 = in1 ? log2_score(x1[ht] * cr[ht] * ks1, lv1) : -INFINITY;
-      float top = fmaxf(s0, s1);
+      float top = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2 * NV; ++j)
+        top = fmaxf(top, fmaxf(fabsf(acc[ht][j][0]), fabsf(acc[ht][j][1])));
 #pragma unroll
       for (int o = 4; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-      top = fmaxf(top, m[ht]);
-      const float base = top == -INFINITY ? 0.f : top - 14.f;  // weights up to 2^14
-      f[ht] = m[ht] == -INFINITY ? 0.f : ex2_approx(m[ht] - top);
-      m[ht] = top;
-      const float w0 = ex2_approx(s0 - base), w1 = ex2_approx(s1 - base);
-      l[ht] = fmaf(l[ht], f[ht], fmaf(w0, iv0, w1 * iv1));
-      pb[ht][0] = transpose_pairs(split_pair(w0));
-      pb[ht][1] = transpose_pairs(split_pair(w1));
+      good &= top >= REFERENCE_WEIGHT || ht * 4 + t >= G;
+      m[ht] -= 14.f;  // the sums are worth 2^m
     }
-    // ---- values ----
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      uint32_t lo[4], hi[4];  // dims 32j + 4g + 0..3 of the first and of the second token pair
-      token_pairs<FP8>(vw[0][j], vw[1][j], lo);
-      token_pairs<FP8>(vw[2][j], vw[3][j], hi);
-#pragma unroll
-      for (int ht = 0; ht < HT; ++ht)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float d4[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_f16(d4, {lo[2 * e], lo[2 * e + 1], hi[2 * e], hi[2 * e + 1]}, pb[ht][0], pb[ht][1]);
-          float(&c)[2] = acc[ht][2 * j + e];
-          c[0] = fmaf(c[0], f[ht], d4[0] + d4[1]);
-          c[1] = fmaf(c[1], f[ht], d4[2] + d4[3]);
-        }
-    }
+    return mine == 0 || __all_sync(0xFFFFFFFFu, good) != 0;
+  };
+  if (!walk(std::false_type{})) {
+    blocks = tile_block(lane);
+    // the newest token's bytes lie in the pool and in a slot: before the copies that read and overwrite them
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncwarp();
+    for (uint32_t i = 0; i < ahead; ++i) load(i, mine + i);
+    walk(std::true_type{});
   }
   // ---- the warps' maxima, sums and accumulators under a common maximum ----
 #pragma unroll
@@ -430,9 +487,9 @@ __global__ void __launch_bounds__(PD_NT, HD == 64 ? 3 : 2)
     float* dst = red + (warp * G + h) * HD + 4 * g;
 #pragma unroll
     for (int j = 0; j < NV; ++j)
-      *reinterpret_cast<float4*>(dst + 32 * j) =
-          make_float4(acc[ht][2 * j][0] * up, acc[ht][2 * j][1] * up, acc[ht][2 * j + 1][0] * up,
-                      acc[ht][2 * j + 1][1] * up);
+      *reinterpret_cast<float4*>(dst + 32 * j) = make_float4(
+          acc[ht][2 * j][0] * up * unit[ht], acc[ht][2 * j][1] * up * unit[ht],
+          acc[ht][2 * j + 1][0] * up * unit[ht], acc[ht][2 * j + 1][1] * up * unit[ht]);
   }
   __syncthreads();
   // warps beyond the partition's tiles have only zeros

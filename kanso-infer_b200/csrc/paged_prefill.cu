@@ -5,25 +5,26 @@
 // that a staged K/V tile of 64 tokens serves 16 rows in each of four warps. The one-row-per-CTA form
 // that decoding uses walks each row's prefix on its own: at 2048 query tokens in four sequences of
 // up to 2240 tokens (15 / 5 heads of 64) that is 2.5 GB of record reads out of L2 and dp4a arithmetic,
-// 838 us with the chunk's store; this form takes 99 us.
+// 838 us with the chunk's store; this form takes 103 us.
 //
 // Numbers, no less exact than the decode form's:
 //   * int8: the query row is two int8 planes (q ~ d (hi + lo / 254)); both products with the int8
 //     K rows are exact int32 sums on m16n8k32. fp8: K as f16 (every E4M3 value is one), the query
 //     row over a power of two as two f16 values.
 //   * V as f16 (exact for both types). The V scale cannot leave the sum over tokens, so it goes into
-//     the weights: w_j = 2^(s_j + log2 vs_j - max), and the softmax's denominator takes w_j / vs_j.
-//     The weights, at most 2^14, go into the products as the sum of two f16 values (22 bits). Only
-//     tokens whose V rows are more than 2^100 smaller than the largest ones lose weight that way.
+//     the weights: w_j = 2^(s_j + log2 vs_j - max), and the softmax's denominator takes w_j / vs_j
+//     (pool_mma.cuh: unless scales are out of the ordinary). The weights, at most 2^14, go into the
+//     products as the sum of two f16 values (22 bits).
 //   * f32 sums, running maximum, one rescaling per tile and only where a maximum moved.
 //
 // Bound: the tensor pipe at mma.sync rates, 8 cycles an instruction per SM quarter (two products for
-// each of Q.K and P.V: 37 us of the 99), and the issue of about 20 instructions per score and lane
+// each of Q.K and P.V: 37 us of the 103), and the issue of about 20 instructions per score and lane
 // of softmax, splitting and matrix loads beside it (38 M instructions, 35 us), which overlap only
 // as far as the three CTAs of an SM are in different phases.
 #include <cuda_fp8.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "kv_pool.h"
 #include "paged_prefill.h"
@@ -60,7 +61,7 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool in) {
                : "memory");
 }
 // Shared memory: raw K and V rows [2][64][HD] each (16-byte chunks swizzled for the matrix loads of
-// K), V as f16 [64][HD] (and K, fp8), the raw scales [2][2][64], the derived ones [3][64].
+// K), V as f16 [64][HD] (and K, fp8), the raw scales [2][2][64], the derived ones [3][64], the unit.
 template <int HD, bool FP8>
 struct PpSmem {
   static constexpr uint32_t raw = PP_TOK * HD;       // one raw tile
@@ -68,7 +69,7 @@ struct PpSmem {
   static constexpr uint32_t v16 = 4 * raw, k16 = v16 + f16;
   static constexpr uint32_t sc = FP8 ? k16 + f16 : k16;
   static constexpr uint32_t der = sc + 4 * PP_TOK * 4;
-  static constexpr uint32_t bytes = der + 3 * PP_TOK * 4;
+  static constexpr uint32_t bytes = der + 3 * PP_TOK * 4 + 16;
 };
 
 template <int HD, bool FP8>
@@ -149,11 +150,13 @@ __global__ void __launch_bounds__(PP_WARPS * 32, HD == 64 ? 3 : 2)
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (i0 < i1) {
+  auto start = [&] {
+    if (i0 >= i1) return;
     find_tile(i0);
     load_tile(i0, 0);
     find_tile(i0 + 1);
-  }
+  };
+  start();
 
   // ---- the query rows as A fragments, two terms each ----
   constexpr int KS = FP8 ? HD / 16 : HD / 32;  // k steps of an instruction
@@ -222,194 +225,260 @@ __global__ void __launch_bounds__(PP_WARPS * 32, HD == 64 ? 3 : 2)
     }
   }
 
-  float o[HD / 8][4];
-#pragma unroll
-  for (int j = 0; j < HD / 8; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-  float mt[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  float o[HD / 8][4], mt[2], l[2], unit[2];  // o counts in units, and is worth 2^mt
   const float* der = reinterpret_cast<const float*>(smem + S::der);
 
-  for (uint32_t i = i0; i < i1; ++i) {
-    const uint32_t st = (i - i0) & 1;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // the tile has landed, and nothing of the one before is still read
-    if (i + 1 < i1) {
-      load_tile(i + 1, st ^ 1);
-      find_tile(i + 2);
+  // All tiles in order; false: a row or token of this thread asks for the careful form.
+  auto walk = [&](auto careful) {
+    constexpr bool CAREFUL = decltype(careful)::value;
+    uint32_t seen = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mt[h] = -INFINITY;
+      l[h] = 0.f;
+      unit[h] = CAREFUL ? 0.f : 1.f;
     }
-    // ---- V (fp8: and K) to f16; scales to what the softmax wants ----
 #pragma unroll
-    for (int w = 0; w < (FP8 ? 2 : 1); ++w) {
+    for (int j = 0; j < HD / 8; ++j)
 #pragma unroll
-      for (int it = 0; it < ITEMS; ++it) {
-        const uint32_t item = tid + it * NT, t = item / CH, c = item % CH;
-        const uint32_t sw = HD == 64 ? c ^ ((t >> 1) & 3) : c ^ (t & 7);
-        const uint4 raw = *reinterpret_cast<const uint4*>(
-            w ? smem + st * S::raw + t * HD + sw * 16 : smem + (2 + st) * S::raw + t * HD + c * 16);
-        const uint2 a0 = bytes_to_f16<FP8>(raw.x), a1 = bytes_to_f16<FP8>(raw.y);
-        const uint2 a2 = bytes_to_f16<FP8>(raw.z), a3 = bytes_to_f16<FP8>(raw.w);
-        uint8_t* d = smem + (w ? S::k16 : S::v16) + t * (HD * 2);
-        *reinterpret_cast<uint4*>(d + (((2 * c) ^ (t & 7)) * 16)) = make_uint4(a0.x, a0.y, a1.x, a1.y);
-        *reinterpret_cast<uint4*>(d + (((2 * c + 1) ^ (t & 7)) * 16)) =
-            make_uint4(a2.x, a2.y, a3.x, a3.y);
+      for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+    for (uint32_t i = i0; i < i1; ++i) {
+      const uint32_t st = (i - i0) & 1;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();  // the tile has landed, and nothing of the one before is still read
+      if (i + 1 < i1) {
+        load_tile(i + 1, st ^ 1);
+        find_tile(i + 2);
       }
-    }
-    if (tid < PP_TOK) {
-      const float* sc = reinterpret_cast<const float*>(smem + S::sc) + st * 2 * PP_TOK;
-      float* d = reinterpret_cast<float*>(smem + S::der);
-      const float vs = fmaxf(sc[PP_TOK + tid], 1.17549435e-38f);
-      d[tid] = sc[tid] * a.scale;
-      d[PP_TOK + tid] = __log2f(vs);
-      d[2 * PP_TOK + tid] = 1.0f / vs;
-    }
-    const bool work = warp_live && (int)(i * PP_TOK) <= wmax;  // the warp has rows that see the tile
-    int sc_i[PP_TOK / 8][4];
-    if (!FP8 && work) {
-      const uint32_t kb = smem_u32(smem + st * S::raw);
+      // ---- V (fp8: and K) to f16; scales to what the softmax wants ----
 #pragma unroll
-      for (int j = 0; j < PP_TOK / 8; ++j) {
-        const uint32_t t = j * 8 + (lane & 7);
-        uint32_t b[KS][2];
+      for (int w = 0; w < (FP8 ? 2 : 1); ++w) {
 #pragma unroll
-        for (int p = 0; p < KS / 2; ++p) {
-          const uint32_t c = p * 4 + (lane >> 3);
+        for (int it = 0; it < ITEMS; ++it) {
+          const uint32_t item = tid + it * NT, t = item / CH, c = item % CH;
           const uint32_t sw = HD == 64 ? c ^ ((t >> 1) & 3) : c ^ (t & 7);
-          uint32_t r[4];
-          ldm_x4(r, kb + t * HD + sw * 16);
-          b[2 * p][0] = r[0];
-          b[2 * p][1] = r[1];
-          b[2 * p + 1][0] = r[2];
-          b[2 * p + 1][1] = r[3];
+          const uint4 raw = *reinterpret_cast<const uint4*>(
+              w ? smem + st * S::raw + t * HD + sw * 16 : smem + (2 + st) * S::raw + t * HD + c * 16);
+          const uint2 a0 = bytes_to_f16<FP8>(raw.x), a1 = bytes_to_f16<FP8>(raw.y);
+          const uint2 a2 = bytes_to_f16<FP8>(raw.z), a3 = bytes_to_f16<FP8>(raw.w);
+          uint8_t* d = smem + (w ? S::k16 : S::v16) + t * (HD * 2);
+          *reinterpret_cast<uint4*>(d + (((2 * c) ^ (t & 7)) * 16)) = make_uint4(a0.x, a0.y, a1.x, a1.y);
+          *reinterpret_cast<uint4*>(d + (((2 * c + 1) ^ (t & 7)) * 16)) =
+              make_uint4(a2.x, a2.y, a3.x, a3.y);
         }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc_i[j][e] = 0;
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks) mma_s8(sc_i[j], qh[ks], b[ks][0], b[ks][1]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc_i[j][e] *= 254;
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks) mma_s8(sc_i[j], ql[ks], b[ks][0], b[ks][1]);
       }
-    }
-    __syncthreads();  // the f16 tiles and the scales are complete
-    if (!work) continue;
-    float t_[PP_TOK / 8][4];
-    if (FP8) {
-      const uint32_t kb = smem_u32(smem + S::k16);
+      if (tid < PP_TOK) {
+        const float* sc = reinterpret_cast<const float*>(smem + S::sc) + st * 2 * PP_TOK;
+        float* d = reinterpret_cast<float*>(smem + S::der);
+        d[tid] = sc[tid] * a.scale;
+        if (CAREFUL) {
+          float vs[2];  // both warps look at the whole tile
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t t = lane + 32 * h;
+            vs[h] = any_value<FP8, CH>(smem + (2 + st) * S::raw + t * HD) ? sc[PP_TOK + t] : 0.f;
+          }
+          const TileUnit tu = tile_unit(vs[0], vs[1]);
+          // finite: rows that do not see a token must not meet its infinite scale
+          d[PP_TOK + tid] = fminf((warp ? vs[1] : vs[0]) * tu.up, 3.4028235e38f);
+          if (tid == 0) d[3 * PP_TOK] = tu.down;
+        } else {
+          const float vs = i * PP_TOK + tid < keys ? sc[PP_TOK + tid] : 1.f;
+          seen |= scale_bits(vs);
+          d[PP_TOK + tid] = __log2f(vs);
+          d[2 * PP_TOK + tid] = 1.0f / vs;
+        }
+      }
+      const bool work = warp_live && (int)(i * PP_TOK) <= wmax;  // the warp has rows that see the tile
+      int sc_i[PP_TOK / 8][4];
+      if (!FP8 && work) {
+        const uint32_t kb = smem_u32(smem + st * S::raw);
+#pragma unroll
+        for (int j = 0; j < PP_TOK / 8; ++j) {
+          const uint32_t t = j * 8 + (lane & 7);
+          uint32_t b[KS][2];
+#pragma unroll
+          for (int p = 0; p < KS / 2; ++p) {
+            const uint32_t c = p * 4 + (lane >> 3);
+            const uint32_t sw = HD == 64 ? c ^ ((t >> 1) & 3) : c ^ (t & 7);
+            uint32_t r[4];
+            ldm_x4(r, kb + t * HD + sw * 16);
+            b[2 * p][0] = r[0];
+            b[2 * p][1] = r[1];
+            b[2 * p + 1][0] = r[2];
+            b[2 * p + 1][1] = r[3];
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc_i[j][e] = 0;
+#pragma unroll
+          for (int ks = 0; ks < KS; ++ks) mma_s8(sc_i[j], qh[ks], b[ks][0], b[ks][1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc_i[j][e] *= 254;
+#pragma unroll
+          for (int ks = 0; ks < KS; ++ks) mma_s8(sc_i[j], ql[ks], b[ks][0], b[ks][1]);
+        }
+      }
+      __syncthreads();  // the f16 tiles and the scales are complete
+      if (!work) continue;
+      float t_[PP_TOK / 8][4];
+      if (FP8) {
+        const uint32_t kb = smem_u32(smem + S::k16);
+#pragma unroll
+        for (int j = 0; j < PP_TOK / 8; ++j) {
+          const uint32_t t = j * 8 + (lane & 7);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) t_[j][e] = 0.f;
+#pragma unroll
+          for (int p = 0; p < KS / 2; ++p) {
+            uint32_t r[4];
+            ldm_x4(r, kb + t * (HD * 2) + (((p * 4 + (lane >> 3)) ^ (t & 7)) * 16));
+            float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_f16(c0, ql[2 * p], r[0], r[1]);
+            mma_f16(c1, ql[2 * p + 1], r[2], r[3]);
+            mma_f16(c0, qh[2 * p], r[0], r[1]);
+            mma_f16(c1, qh[2 * p + 1], r[2], r[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) t_[j][e] += c0[e] + c1[e];
+          }
+        }
+      }
+      // ---- scores in units of log2, with the V scale's logarithm ----
+      float top[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int j = 0; j < PP_TOK / 8; ++j) {
-        const uint32_t t = j * 8 + (lane & 7);
+        const float2 ks2 = *reinterpret_cast<const float2*>(der + j * 8 + (lane & 3) * 2);
+        const float2 lv2 = *reinterpret_cast<const float2*>(der + PP_TOK + j * 8 + (lane & 3) * 2);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) t_[j][e] = 0.f;
-#pragma unroll
-        for (int p = 0; p < KS / 2; ++p) {
-          uint32_t r[4];
-          ldm_x4(r, kb + t * (HD * 2) + (((p * 4 + (lane >> 3)) ^ (t & 7)) * 16));
-          float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_f16(c0, ql[2 * p], r[0], r[1]);
-          mma_f16(c1, ql[2 * p + 1], r[2], r[3]);
-          mma_f16(c0, qh[2 * p], r[0], r[1]);
-          mma_f16(c1, qh[2 * p + 1], r[2], r[3]);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) t_[j][e] += c0[e] + c1[e];
+        for (int e = 0; e < 4; ++e) {
+          const float x = FP8 ? t_[j][e] : (float)sc_i[j][e];
+          const float u = x * cr[e >> 1] * ((e & 1) ? ks2.y : ks2.x);
+          t_[j][e] = CAREFUL ? log2_units(u) : log2_score(u, (e & 1) ? lv2.y : lv2.x);
         }
       }
-    }
-    // ---- scores in units of log2, with the V scale's logarithm ----
-    float top[2] = {-INFINITY, -INFINITY};
+      if ((int)(i * PP_TOK + PP_TOK - 1) > wmin) {  // some row of the warp does not see all of it
 #pragma unroll
-    for (int j = 0; j < PP_TOK / 8; ++j) {
-      const float2 ks2 = *reinterpret_cast<const float2*>(der + j * 8 + (lane & 3) * 2);
-      const float2 lv2 = *reinterpret_cast<const float2*>(der + PP_TOK + j * 8 + (lane & 3) * 2);
+        for (int j = 0; j < PP_TOK / 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float x = FP8 ? t_[j][e] : (float)sc_i[j][e];
-        t_[j][e] = log2_score(x * cr[e >> 1] * ((e & 1) ? ks2.y : ks2.x),
-                              (e & 1) ? lv2.y : lv2.x);
+          for (int e = 0; e < 4; ++e)
+            if ((int)(i * PP_TOK + j * 8 + (lane & 3) * 2 + (e & 1)) > lim[e >> 1])
+              t_[j][e] = -INFINITY;
       }
-    }
-    if ((int)(i * PP_TOK + PP_TOK - 1) > wmin) {  // some row of the warp does not see all of it
 #pragma unroll
-      for (int j = 0; j < PP_TOK / 8; ++j)
+      for (int j = 0; j < PP_TOK / 8; ++j) {
+        top[0] = fmaxf(top[0], fmaxf(t_[j][0], t_[j][1]));
+        top[1] = fmaxf(top[1], fmaxf(t_[j][2], t_[j][3]));
+      }
+      float base[2];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if ((int)(i * PP_TOK + j * 8 + (lane & 3) * 2 + (e & 1)) > lim[e >> 1])
-            t_[j][e] = -INFINITY;
-    }
+      for (int h = 0; h < 2; ++h) {
+        top[h] = fmaxf(top[h], __shfl_xor_sync(0xFFFFFFFFu, top[h], 1));
+        top[h] = fmaxf(top[h], __shfl_xor_sync(0xFFFFFFFFu, top[h], 2));
+        // a whole number in the careful form, whose later changes to the reference are then exact
+        top[h] = fmaxf(CAREFUL ? ceilf(top[h]) : top[h], mt[h]);
+        base[h] = top[h] == -INFINITY ? 0.f : CAREFUL ? top[h] : top[h] - 14.f;  // weights up to 2^14
+      }
+      float f[2];  // what the earlier sums are worth under the new maximum
 #pragma unroll
-    for (int j = 0; j < PP_TOK / 8; ++j) {
-      top[0] = fmaxf(top[0], fmaxf(t_[j][0], t_[j][1]));
-      top[1] = fmaxf(top[1], fmaxf(t_[j][2], t_[j][3]));
-    }
-    float base[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      top[h] = fmaxf(top[h], __shfl_xor_sync(0xFFFFFFFFu, top[h], 1));
-      top[h] = fmaxf(top[h], __shfl_xor_sync(0xFFFFFFFFu, top[h], 2));
-      top[h] = fmaxf(top[h], mt[h]);
-      base[h] = top[h] == -INFINITY ? 0.f : top[h] - 14.f;  // weights up to 2^14
-    }
-    float f[2];  // what the earlier sums are worth under the new maximum
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      f[h] = mt[h] == -INFINITY ? 0.f : ex2_approx(mt[h] - top[h]);
-      l[h] *= f[h];
-      mt[h] = top[h];
-    }
-    // ---- weights and their sums ----
-    uint32_t ph[PP_TOK / 16][4], pl[PP_TOK / 16][4];
-#pragma unroll
-    for (int k = 0; k < PP_TOK / 16; ++k) {
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {  // tokens 16k + 8p ..
-        const int j = 2 * k + p;
-        const float2 iv = *reinterpret_cast<const float2*>(der + 2 * PP_TOK + j * 8 + (lane & 3) * 2);
+      for (int h = 0; h < 2; ++h) {
+        f[h] = mt[h] == -INFINITY ? 0.f : ex2_approx(mt[h] - top[h]);
+        l[h] *= f[h];
+        mt[h] = top[h];
+      }
+      float own[2] = {1.f, 1.f};  // careful: what the exponentials' sums are worth
+      if (CAREFUL) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const float w0 = ex2_approx(t_[j][2 * h] - base[h]);
-          const float w1 = ex2_approx(t_[j][2 * h + 1] - base[h]);
-          l[h] = fmaf(w0, iv.x, l[h]);
-          l[h] = fmaf(w1, iv.y, l[h]);
-          split_f16(w0, w1, ph[k][p * 2 + h], pl[k][p * 2 + h]);
+          float largest = 0.f;
+#pragma unroll
+          for (int j = 0; j < PP_TOK / 8; ++j) {
+            const float* vn = der + PP_TOK + j * 8 + (lane & 3) * 2;
+            largest = fmaxf(largest, ex2_approx(t_[j][2 * h] - base[h]) * vn[0]);
+            largest = fmaxf(largest, ex2_approx(t_[j][2 * h + 1] - base[h]) * vn[1]);
+          }
+          largest = fmaxf(largest, __shfl_xor_sync(0xFFFFFFFFu, largest, 1));
+          largest = fmaxf(largest, __shfl_xor_sync(0xFFFFFFFFu, largest, 2));
+          const int by = lift_weights(largest, der[3 * PP_TOK], f[h], unit[h]);
+          base[h] -= (float)by;
+          own[h] = exp2i(-by);
         }
       }
-    }
-    // ---- the tile's product with V, added to the sums outside of the tensor cores: those cut
-    // off where an f32 addition rounds, which over hundreds of steps is a bias of 3e-6 ----
-    const uint32_t vb = smem_u32(smem + S::v16);
-#pragma unroll
-    for (int d = 0; d < HD / 16; ++d) {
-      float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+      // ---- weights and their sums ----
+      uint32_t ph[PP_TOK / 16][4], pl[PP_TOK / 16][4];
 #pragma unroll
       for (int k = 0; k < PP_TOK / 16; ++k) {
-        const uint32_t t = k * 16 + (lane & 15);
-        uint32_t r[4];
-        ldm_x4_t(r, vb + t * (HD * 2) + (((2 * d + (lane >> 4)) ^ (t & 7)) * 16));
-        if (FP8) {  // sums of 16 tokens there (and of 32 dims above): 3e-7 against 4.6e-7 of 64
-          float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_f16(c0, pl[k], r[0], r[1]);
-          mma_f16(c1, pl[k], r[2], r[3]);
-          mma_f16(c0, ph[k], r[0], r[1]);
-          mma_f16(c1, ph[k], r[2], r[3]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s0[e] += c0[e];
-            s1[e] += c1[e];
+        for (int p = 0; p < 2; ++p) {  // tokens 16k + 8p ..
+          const int j = 2 * k + p;
+          const float2 iv = *reinterpret_cast<const float2*>(
+              der + (CAREFUL ? 1 : 2) * PP_TOK + j * 8 + (lane & 3) * 2);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float w0 = ex2_approx(t_[j][2 * h] - base[h]);
+            float w1 = ex2_approx(t_[j][2 * h + 1] - base[h]);
+            l[h] = fmaf(w0, CAREFUL ? own[h] : iv.x, l[h]);
+            l[h] = fmaf(w1, CAREFUL ? own[h] : iv.y, l[h]);
+            if (CAREFUL) {
+              w0 *= iv.x;
+              w1 *= iv.y;
+            }
+            split_f16(w0, w1, ph[k][p * 2 + h], pl[k][p * 2 + h]);
           }
-        } else {
-          mma_f16(s0, pl[k], r[0], r[1]);
-          mma_f16(s1, pl[k], r[2], r[3]);
-          mma_f16(s0, ph[k], r[0], r[1]);
-          mma_f16(s1, ph[k], r[2], r[3]);
         }
       }
+      // ---- the tile's product with V, added to the sums outside of the tensor cores: those cut
+      // off where an f32 addition rounds, which over hundreds of steps is a bias of 3e-6 ----
+      const uint32_t vb = smem_u32(smem + S::v16);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        o[2 * d][e] = fmaf(o[2 * d][e], f[e >> 1], s0[e]);
-        o[2 * d + 1][e] = fmaf(o[2 * d + 1][e], f[e >> 1], s1[e]);
+      for (int d = 0; d < HD / 16; ++d) {
+        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < PP_TOK / 16; ++k) {
+          const uint32_t t = k * 16 + (lane & 15);
+          uint32_t r[4];
+          ldm_x4_t(r, vb + t * (HD * 2) + (((2 * d + (lane >> 4)) ^ (t & 7)) * 16));
+          if (FP8) {  // sums of 16 tokens there (and of 32 dims above): 3e-7 against 4.6e-7 of 64
+            float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_f16(c0, pl[k], r[0], r[1]);
+            mma_f16(c1, pl[k], r[2], r[3]);
+            mma_f16(c0, ph[k], r[0], r[1]);
+            mma_f16(c1, ph[k], r[2], r[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              s0[e] += c0[e];
+              s1[e] += c1[e];
+            }
+          } else {
+            mma_f16(s0, pl[k], r[0], r[1]);
+            mma_f16(s1, pl[k], r[2], r[3]);
+            mma_f16(s0, ph[k], r[0], r[1]);
+            mma_f16(s1, ph[k], r[2], r[3]);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          o[2 * d][e] = fmaf(o[2 * d][e], f[e >> 1], s0[e]);
+          o[2 * d + 1][e] = fmaf(o[2 * d + 1][e], f[e >> 1], s1[e]);
+        }
       }
     }
+
+    bool good = CAREFUL || !unusual_scales(seen);
+#pragma unroll
+    for (int h = 0; h < 2 && !CAREFUL; ++h) {
+      float top = 0.f;
+#pragma unroll
+      for (int j = 0; j < HD / 8; ++j)
+        top = fmaxf(top, fmaxf(fabsf(o[j][2 * h]), fabsf(o[j][2 * h + 1])));
+      top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
+      top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
+      good &= top >= REFERENCE_WEIGHT || mt[h] == -INFINITY;
+      mt[h] -= 14.f;
+    }
+    return good;
+  };
+  if (__syncthreads_or(!walk(std::false_type{}))) {
+    start();
+    walk(std::true_type{});
   }
 
 #pragma unroll
@@ -424,7 +493,7 @@ __global__ void __launch_bounds__(PP_WARPS * 32, HD == 64 ? 3 : 2)
 #pragma unroll
     for (int j = 0; j < HD / 8; ++j)
       *reinterpret_cast<float2*>(dst + j * 8 + (lane & 3) * 2) =
-          make_float2(o[j][2 * h] * inv, o[j][2 * h + 1] * inv);
+          make_float2(o[j][2 * h] * inv * unit[h], o[j][2 * h + 1] * inv * unit[h]);
     if (a.splits > 1 && (lane & 3) == 0)
       *reinterpret_cast<float2*>(a.part + a.splits * all * HD + (split * all + row) * 2) =
           make_float2(mt[h], l[h]);

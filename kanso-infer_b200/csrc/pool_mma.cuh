@@ -63,6 +63,62 @@ __device__ __forceinline__ void pow2_scale(float top, float& up, float& down) {
 __device__ __forceinline__ float log2_score(float u, float lv) {
   return fmaf(u, 1.44269502f, fmaf(u, 1.92596303e-8f, lv));
 }
+// u * log2(e) alone.
+__device__ __forceinline__ float log2_units(float u) {
+  return fmaf(u, 1.44269502f, u * 1.92596303e-8f);
+}
+
+// ---- V scales ----
+// The V scale cannot leave the sum over tokens. The kernels take it into the weight, w = 2^(s + log2 vs - max),
+// so that the largest contribution is the reference of the two f16 values (22 bits, down to 2^-38 of it),
+// and add w / vs to the denominator. That is exact enough if scales are far from the ends of f32 and the
+// reference does contribute; a row of zeros, stored with the scale 1, does not, and may outweigh rows
+// that are far smaller. Both show at the end of a pass: some scale was outside of 2^-32 to 2^32, or no
+// element of the sums reaches 2^14, the reference's weight (its largest value is 32 or more). Then the
+// pass is made once more in the careful form: exponentials of the score alone, which the denominator adds;
+// scales relative to the tile's largest; weights brought up tile by tile (lift_weights), sums in units
+// of the largest weight so far.
+constexpr float REFERENCE_WEIGHT = 16384.f;
+// Bits above 28 in the union of these over all scales: one was unusual. Tests of every scale and row as they
+// pass took 4 % of both kernels' time; this and the look at the sums 3 % of the prompt kernel's (2048
+// query tokens, 15 / 5 heads of 64: 100 -> 103 us) and nothing of the decode kernel's at head size 64.
+__device__ __forceinline__ uint32_t scale_bits(float v) { return __float_as_uint(v) - (95u << 23); }
+__device__ __forceinline__ bool unusual_scales(uint32_t bits) { return bits >> 29; }
+// Whether the 16 N bytes at p hold any value but zero (E4M3 has a second one).
+template <bool FP8, int N>
+__device__ __forceinline__ bool any_value(const uint8_t* p) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p + 16 * i);
+    o |= v.x | v.y | v.z | v.w;
+  }
+  return (o & (FP8 ? 0x7F7F7F7Fu : ~0u)) != 0;
+}
+// Careful form, all lanes of a warp: the power of two that brings the lanes' scales (0 for no row or a
+// row of zeros) under 2^14, and its inverse, which is a normal number.
+struct TileUnit {
+  float up, down;
+};
+__device__ __forceinline__ TileUnit tile_unit(float v0, float v1) {
+  const uint32_t top =
+      __reduce_max_sync(0xFFFFFFFFu, max(__float_as_uint(v0), __float_as_uint(v1))) >> 23;
+  const uint32_t e = min(max(top, 14u), 254u);
+  return {__uint_as_float((267u - e) << 23), __uint_as_float((e - 13u) << 23)};
+}
+__device__ __forceinline__ float exp2i(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
+// The logarithm of the power of two that brings weights up whose largest is `top`, in units of `down`: to
+// under 2^14, or to the unit of the earlier sums if those are the larger ones. f: what the earlier sums
+// are worth under the new maximum, made their factor; unit: theirs, made the new one.
+__device__ __forceinline__ int lift_weights(float top, float down, float& f, float& unit) {
+  const int d = (int)(__float_as_uint(down) >> 23);
+  const int by = max(min(140 - max((int)(__float_as_uint(top) >> 23), 40), d - 1), 0);
+  const float least = __uint_as_float((uint32_t)(d - by) << 23), before = unit * f;
+  const int b = (int)(__float_as_uint(before) >> 23) + 1;
+  unit = before > least ? __uint_as_float((uint32_t)b << 23) : least;
+  f = before / unit;
+  return before > least ? max(d - b, -100) : by;
+}
 // x as two f16 values, side by side
 __device__ __forceinline__ uint32_t split_pair(float x) {
   const __half h = __float2half_rn(x);
