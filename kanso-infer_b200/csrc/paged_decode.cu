@@ -510,7 +510,9 @@ uint32_t pa_mma_partition_tokens(const kanso_cuda_ctx* ctx, const kanso_paged_at
          (uint64_t)p->num_seqs * p->num_kv_heads * ((cap + pt - 1) / pt) <
              2 * (uint64_t)ctx->sm_count)
     pt >>= 1;
-  return (pt + g.block_size - 1) / g.block_size * g.block_size;
+  pt = (pt + g.block_size - 1) / g.block_size * g.block_size;
+  // partitions lie along the grid's third dimension (a table of 134 million tokens, no host lengths)
+  return (cap + pt - 1) / pt > 65535 ? 0 : pt;
 }
 
 template <int G, bool FP8, int HD>

@@ -51,3 +51,28 @@ def test_paged_decode_edges(ctx, kb, oracle, torch_cuda, pool, H, KH, hd, bs):
     got = out.cpu().numpy()
     for i in range(len(lens)):
         assert rel_err(got[i], ref[i]) <= (2e-5 if pool == "fp8" else 1e-4), lens[i]
+
+
+def test_table_of_more_partitions_than_a_grid_holds(ctx, kb, torch_cuda):
+    """Without lengths on the host the grid covers the whole table: 65,536 partitions of 2048 tokens are
+    more than the grid's third dimension holds, which the general kernel's first does."""
+    torch = torch_cuda
+    bs, hd, lens = 1024, 64, np.array([37], np.uint32)
+    maxb = 65536 * 2048 // bs
+    rng = np.random.Generator(np.random.PCG64(0xB2000D80))
+    gp = kb.KvPool(ctx, 1, 1, bs, 1, hd, kb.KV_INT8)
+    k, v = (torch.from_numpy(rng.standard_normal((37, hd)).astype(np.float32)).cuda()
+            for _ in range(2))
+    gp.write_slots(0, torch.arange(37, dtype=torch.int32, device="cuda"), k, v, 37)
+    q = torch.from_numpy(rng.standard_normal((1, hd)).astype(np.float32)).cuda()
+    tab = torch.zeros(maxb, dtype=torch.int32, device="cuda")
+    ln = torch.from_numpy(lens.astype(np.int32)).cuda()
+    outs = []
+    for blocks, host in ((1, lens), (maxb, None)):
+        out = torch.full((1, hd), float("nan"), device="cuda")
+        gp.paged_attention(0, q, tab, ln, out,
+                           kb.PagedAttentionParams(1, 1, 1, hd, bs, blocks, hd ** -0.5), host)
+        ctx.sync()
+        outs.append(out.cpu().numpy())
+    assert rel_err(outs[1], outs[0]) <= 1e-4
+    gp.destroy()
