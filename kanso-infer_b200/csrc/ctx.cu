@@ -24,6 +24,7 @@ int32_t fail(kanso_cuda_ctx* ctx, int32_t code, const char* fmt, ...) {
 }
 
 int32_t cuda_fail(kanso_cuda_ctx* ctx, cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next launch's check must not find it
   return fail(ctx, KANSO_ERR_DEVICE, "%s: %s (%s)", what, cudaGetErrorString(e),
               cudaGetErrorName(e));
 }

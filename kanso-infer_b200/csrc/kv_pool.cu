@@ -119,6 +119,7 @@ int32_t kanso_cuda_kv_create(kanso_cuda_ctx* ctx, uint32_t num_layers, uint32_t 
   cudaError_t e = cudaMalloc((void**)&kv->pool, kv->pool_bytes);
   if (e != cudaSuccess) {
     delete kv;
+    cudaGetLastError();
     // an allocation failure at start-up is a Config error (src/kv_cache/storage.rs:29-68)
     return fail(ctx, KANSO_ERR_CONFIG, "kv_create: cannot allocate %zu bytes of KV pool: %s",
                 (size_t)num_layers * num_blocks * num_kv_heads * g.rec_bytes,
