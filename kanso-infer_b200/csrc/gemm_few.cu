@@ -578,9 +578,10 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   int nt = (int)(M + 7) / 8, grid = 0;
   if (int8) {
     // Whole rows per CTA (results bit-identical to the CPU's) while the tiles fill the GPU; fewer
-    // tiles are split along K while the grid stays within about one wave.
+    // tiles are split along K while the grid stays within about one wave and every part keeps two
+    // units: K below 1024 stays whole whatever the number of rows.
     int split = 1;
-    while (tiles * split * 2 <= ctx->sm_count + ctx->sm_count / 4 && chunks / (split * 2) >= 1)
+    while (tiles * split * 2 <= ctx->sm_count + ctx->sm_count / 4 && chunks / (split * 2) >= 2)
       split *= 2;
     grid = (int)tiles * split;
     a.add = split > 1;

@@ -61,3 +61,55 @@ def test_few_rows_q8_activations(ctx, kb, oracle, torch_cuda, M, N, K):
     for shift in (0, 3):
         got = run(ctx, kb, torch_cuda, kb.DTYPE_Q8_0, blocks, x, N, kb.ACT_Q8, shift)
         assert rel_err(got, ref) <= 1e-5
+
+
+def matrix(fmt, N, K):
+    """Random blocks [N x K] of ordinary size, and their bytes per row."""
+    rng = np.random.Generator(np.random.PCG64(0xB2000C80 + N + K))
+    if fmt == "q8_0":
+        b = rng.integers(0, 256, (N, K // 32, 34), dtype=np.uint8)
+        b[..., :2] = (rng.uniform(0.5, 2, (N, K // 32, 1)) * 1e-4).astype(np.float16).view(np.uint8)
+    else:
+        b = rng.integers(0, 256, (N, K // 256, 144), dtype=np.uint8)
+        b[..., :2] = (rng.uniform(0.5, 2, (N, K // 256, 1)) * 1e-4).astype(np.float16).view(np.uint8)
+        b[..., 2:4] = (rng.uniform(3, 12, (N, K // 256, 1)) * 1e-4).astype(np.float16).view(np.uint8)
+    return b.reshape(N, -1)
+
+
+def some_rows(N):
+    edges = [0, 1, 111, 112, 127, 128, N - 129, N - 113, N - 2, N - 1]
+    return np.unique(edges + list(range(5, N, N // 40)))
+
+
+def several_calls(ctx, kb, torch, fmt, blocks, x, N, act, calls=4):
+    """The result of every one of `calls` calls, behind one another on the stream."""
+    M, K = x.shape
+    w, xd = torch.from_numpy(blocks).cuda(), torch.from_numpy(x).cuda()
+    ys = [torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda") for _ in range(calls)]
+    torch.cuda.synchronize()
+    for y in ys:
+        (ctx.gemm_q8_0 if fmt == "q8_0" else ctx.gemm_q4_k)(w, xd, y, M, N, K, act)
+    ctx.sync()
+    return [y.cpu().numpy() for y in ys]
+
+
+# Matrices whose K stays whole: 93 tiles of 112 rows, and a K of fewer than four units
+@pytest.mark.parametrize("M,N,K", [(24, 10400, 2048), (48, 10400, 2048), (64, 10400, 2048),
+                                   (96, 10400, 2048),
+                                   (16, 1000, 512), (128, 300, 768), (9, 131, 256)])
+def test_q8_activations_bit_exact(ctx, kb, oracle, torch_cuda, M, N, K):
+    blocks = matrix("q8_0", N, K)
+    x = data(M, 1, K)[1]
+    got = several_calls(ctx, kb, torch_cuda, "q8_0", blocks, x, N, kb.ACT_Q8, 1)[0]
+    pick = some_rows(N)
+    ref = oracle.gemm_q8_0(np.ascontiguousarray(blocks[pick]).reshape(-1), x, M, pick.size, K,
+                           oracle.ACT_Q8)
+    assert (got[:, pick] == ref).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 8000, 2048), (33, 2048, 1280)])
+def test_q8_activations_halved_k_repeats(ctx, kb, oracle, torch_cuda, M, N, K):
+    blocks = matrix("q8_0", N, K)
+    got = several_calls(ctx, kb, torch_cuda, "q8_0", blocks, data(M, 1, K)[1], N, kb.ACT_Q8)
+    for again in got[1:]:
+        assert (got[0] == again).all()
