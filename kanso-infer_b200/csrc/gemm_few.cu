@@ -9,7 +9,7 @@
 // hundred rows. mma.sync reaches 1024 (f16) and 2048 (int8) multiply-adds per clock and SM here,
 // which is enough up to about 64 rows.
 //
-//   * A unit is 128 weight rows (int8 form: 112) x 256 k: one tensor-map copy of 272 (Q8_0) or 144
+//   * A unit is 128 weight rows (int8 form: 128 or 112) x 256 k: one tensor-map copy of 272 (Q8_0) or 144
 //     (Q4_K) bytes a row, whole blocks, in rows whose stride is 16 bytes past a multiple of 128, so that
 //     8 rows x 4 lanes of 4-byte reads meet 32 different banks without a swizzle.
 //   * Units are numbered tile by tile and dealt out in equal contiguous runs; the runs ignore tile
@@ -41,13 +41,6 @@ enum FewForm { FEW_Q8_F16, FEW_Q4_F16, FEW_Q8_INT8 };
 constexpr int FEW_K = 256;     // k of a unit
 constexpr int FEW_MAX_STAGES = 6;
 
-// Weight rows of a unit. INT8: whole rows of K per CTA, bound by the arithmetic of the SMs that have
-// one: 112 rows give a matrix of 14336 rows to 128 SMs where 128 rows give it to 112 (128 activation
-// rows 106 -> 100 us, 4096 x 14336 99 -> 95 us).
-template <int FORM>
-__host__ __device__ constexpr int few_tile() {
-  return FORM == FEW_Q8_INT8 ? 112 : 128;
-}
 template <int FORM>
 __host__ __device__ constexpr int few_row_bytes() {  // of one weight row in a unit
   return FORM == FEW_Q4_F16 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES;
@@ -362,12 +355,12 @@ __device__ __forceinline__ void few_unit_int8(float (&acc)[RT][NT][4], const uin
 // their sums meet in shared memory before they leave the CTA) or the activation rows (INT8: groups
 // of NT x 8). No wait is unbounded: after one that ran out a warp skips its work but still takes
 // part in the barriers of its row group.
-template <int FORM, int RT, int NT, int OTHER, int CTAS>
-__global__ void __launch_bounds__(few_tile<FORM>() / (16 * RT) * OTHER * 32 + 32, CTAS)
+template <int FORM, int TILE, int RT, int NT, int OTHER, int CTAS>
+__global__ void __launch_bounds__(TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
     gemm_few_kernel(const __grid_constant__ CUtensorMap tmap, const FewArgs a) {
-  constexpr int WR = few_tile<FORM>() / (16 * RT), WARPS = WR * OTHER;
+  constexpr int WR = TILE / (16 * RT), WARPS = WR * OTHER;
   constexpr int Mp = NT * 8 * (FORM == FEW_Q8_INT8 ? OTHER : 1);
-  constexpr uint32_t W_BYTES = few_tile<FORM>() * few_row_bytes<FORM>();
+  constexpr uint32_t W_BYTES = TILE * few_row_bytes<FORM>();
   constexpr uint32_t X_BYTES = Mp * few_x_bytes<FORM>();
   constexpr uint32_t STAGE = W_BYTES + X_BYTES;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -393,7 +386,7 @@ __global__ void __launch_bounds__(few_tile<FORM>() / (16 * RT) * OTHER * 32 + 32
       auto weights = [&](int u, int slot) {
         mbar_arrive_expect_tx(&full[slot], STAGE);
         tma_load_2d(smem + slot * STAGE, &tmap, u % a.chunks * (few_row_bytes<FORM>() / 4),
-                    u / a.chunks * few_tile<FORM>(), &full[slot]);
+                    u / a.chunks * TILE, &full[slot]);
       };
       auto rows = [&](int u, int slot) {
         bulk_g2s(smem + slot * STAGE + W_BYTES, a.xp + (int64_t)(u % a.chunks) * X_BYTES, X_BYTES,
@@ -466,7 +459,7 @@ __global__ void __launch_bounds__(few_tile<FORM>() / (16 * RT) * OTHER * 32 + 32
         asm volatile("bar.sync %0, %1;" ::"r"(1 + wr), "n"(OTHER * 32) : "memory");
       }
     }
-    const int64_t n0 = (int64_t)(u / a.chunks) * few_tile<FORM>() + wr * (16 * RT) + g;
+    const int64_t n0 = (int64_t)(u / a.chunks) * TILE + wr * (16 * RT) + g;
     const int m0 = (FORM == FEW_Q8_INT8 ? other * NT * 8 : 0) + 2 * t;
     if (ok && (FORM == FEW_Q8_INT8 || other == 0))
 #pragma unroll
@@ -498,11 +491,11 @@ __global__ void __launch_bounds__(few_tile<FORM>() / (16 * RT) * OTHER * 32 + 32
   if (!ok && lane == 0) atomicOr(a.status, DEV_WAIT_TIMEOUT);
 }
 
-template <int FORM, int RT, int NT, int OTHER, int CTAS>
+template <int FORM, int TILE, int RT, int NT, int OTHER, int CTAS>
 static int32_t few_launch(kanso_cuda_ctx* ctx, const CUtensorMap& map, FewArgs a, int grid) {
-  constexpr int WR = few_tile<FORM>() / (16 * RT);
+  constexpr int WR = TILE / (16 * RT);
   constexpr int Mp = NT * 8 * (FORM == FEW_Q8_INT8 ? OTHER : 1);
-  constexpr size_t stage = few_tile<FORM>() * few_row_bytes<FORM>() + Mp * few_x_bytes<FORM>();
+  constexpr size_t stage = TILE * few_row_bytes<FORM>() + Mp * few_x_bytes<FORM>();
   constexpr size_t slab =
       FORM == FEW_Q8_INT8 ? 0 : (OTHER - 1) * WR * RT * (NT < 2 ? NT : 2) * 4 * 32 * 4;
   // CTAS blocks share an SM's memory, of which each needs 1 KB besides and its static part
@@ -512,7 +505,7 @@ static int32_t few_launch(kanso_cuda_ctx* ctx, const CUtensorMap& map, FewArgs a
   if (stages > FEW_MAX_STAGES) stages = FEW_MAX_STAGES;
   if (stages < 2) return fail(ctx, KANSO_ERR_UNSUPPORTED, "gemm_few: no room for two stages");
   a.stages = stages;
-  auto kern = gemm_few_kernel<FORM, RT, NT, OTHER, CTAS>;
+  auto kern = gemm_few_kernel<FORM, TILE, RT, NT, OTHER, CTAS>;
   const int32_t st = allow_max_smem(ctx, (const void*)kern);
   if (st) return st;
   prefer_max_shared(ctx, (const void*)kern);
@@ -528,13 +521,46 @@ template <int FORM>
 static int32_t few_launch_f16(kanso_cuda_ctx* ctx, int nt, const CUtensorMap& map,
                               const FewArgs& a) {
   switch (nt) {
-    case 1: return few_launch<FORM, 2, 1, 2, 2>(ctx, map, a, 0);
-    case 2: return few_launch<FORM, 2, 2, 2, 2>(ctx, map, a, 0);
-    case 3: return few_launch<FORM, 2, 3, 2, 2>(ctx, map, a, 0);
-    case 4: return few_launch<FORM, 2, 4, 2, 2>(ctx, map, a, 0);
-    case 6: return few_launch<FORM, 2, 6, 2, 1>(ctx, map, a, 0);
-    default: return few_launch<FORM, 2, 8, 2, 1>(ctx, map, a, 0);
+    case 1: return few_launch<FORM, 128, 2, 1, 2, 2>(ctx, map, a, 0);
+    case 2: return few_launch<FORM, 128, 2, 2, 2, 2>(ctx, map, a, 0);
+    case 3: return few_launch<FORM, 128, 2, 3, 2, 2>(ctx, map, a, 0);
+    case 4: return few_launch<FORM, 128, 2, 4, 2, 2>(ctx, map, a, 0);
+    case 6: return few_launch<FORM, 128, 2, 6, 2, 1>(ctx, map, a, 0);
+    default: return few_launch<FORM, 128, 2, 8, 2, 1>(ctx, map, a, 0);
   }
+}
+
+template <int TILE>
+static int32_t few_launch_int8(kanso_cuda_ctx* ctx, int nt, const CUtensorMap& map,
+                               const FewArgs& a, int grid) {
+  switch (nt) {
+    case 2: return few_launch<FEW_Q8_INT8, TILE, 1, 2, 1, 1>(ctx, map, a, grid);
+    case 3: return few_launch<FEW_Q8_INT8, TILE, 1, 3, 1, 1>(ctx, map, a, grid);
+    case 4: return few_launch<FEW_Q8_INT8, TILE, 1, 4, 1, 1>(ctx, map, a, grid);
+    case 6: return few_launch<FEW_Q8_INT8, TILE, 1, 3, 2, 1>(ctx, map, a, grid);
+    case 8: return few_launch<FEW_Q8_INT8, TILE, 1, 4, 2, 1>(ctx, map, a, grid);
+  }
+  // 128 weight rows leave no room for four warps to a row group (1056 threads)
+  constexpr int O = TILE == 128 ? 2 : 4;
+  return nt == 12 ? few_launch<FEW_Q8_INT8, TILE, 1, 12 / O, O, 1>(ctx, map, a, grid)
+                  : few_launch<FEW_Q8_INT8, TILE, 1, 16 / O, O, 1>(ctx, map, a, grid);
+}
+
+// How an int8 product is shared out: whole rows per CTA (results bit-identical to the CPU's) while the
+// tiles fill the GPU; fewer tiles are split along K while the grid stays within about one wave and
+// every part keeps two units (K below 1024 stays whole whatever the number of rows).
+struct FewShare {
+  int tile, split;
+  int64_t tiles, chain;  // chain: weight rows x units that the busiest SM goes through
+};
+static FewShare few_share(const kanso_cuda_ctx* ctx, int tile, int64_t N, int64_t chunks) {
+  FewShare s = {tile, 1, (N + tile - 1) / tile, 0};
+  while (s.tiles * s.split * 2 <= ctx->sm_count + ctx->sm_count / 4 &&
+         chunks / (s.split * 2) >= 2)
+    s.split *= 2;
+  const int64_t waves = (s.tiles * s.split + ctx->sm_count - 1) / ctx->sm_count;
+  s.chain = waves * tile * ((chunks + s.split - 1) / s.split);
+  return s;
 }
 
 // y[M,N] = x[M,K] @ W^T for up to 64 activation rows in f16 (act_mode F32) or 128 in exact int8
@@ -549,8 +575,15 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   if (M < 1 || M > (int8 ? 128 : 64) || N < 1 || K < FEW_K || K % FEW_K != 0 || !w || !x || !y)
     return KANSO_OK;
   const int64_t row_bytes = K / FEW_K * (q4 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES);
-  const int tile = int8 ? few_tile<FEW_Q8_INT8>() : few_tile<FEW_Q8_F16>();
-  const int64_t chunks = K / FEW_K, tiles = (N + tile - 1) / tile;
+  const int64_t chunks = K / FEW_K;
+  // The int8 form is bound by the arithmetic of the SMs that have any: tiles of 112 rows where they
+  // shorten the longest chain of rows on an SM. us at 128 activation rows with 112 and with 128:
+  // 14336 x 4096 (128 and 112 busy SMs) 100 and 106 with cold caches; 17408 x 4096, two waves of 112 rows
+  // and one of 128, 130 and 72 behind one another, 18944 x 3584 115 and 64.
+  const FewShare s128 = few_share(ctx, 128, N, chunks), s112 = few_share(ctx, 112, N, chunks);
+  const FewShare& share = int8 && s112.chain < s128.chain ? s112 : s128;
+  const int tile = share.tile;
+  const int64_t tiles = share.tiles;
   if (!aligned16(w) || row_bytes > (1 << 28) || tiles * chunks > (1 << 30) || N > (1 << 30))
     return KANSO_OK;
   TmEncodeFn encode = tm_encoder();
@@ -577,14 +610,8 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   a.status = ctx->dev_status;
   int nt = (int)(M + 7) / 8, grid = 0;
   if (int8) {
-    // Whole rows per CTA (results bit-identical to the CPU's) while the tiles fill the GPU; fewer
-    // tiles are split along K while the grid stays within about one wave and every part keeps two
-    // units: K below 1024 stays whole whatever the number of rows.
-    int split = 1;
-    while (tiles * split * 2 <= ctx->sm_count + ctx->sm_count / 4 && chunks / (split * 2) >= 2)
-      split *= 2;
-    grid = (int)tiles * split;
-    a.add = split > 1;
+    grid = (int)tiles * share.split;
+    a.add = share.split > 1;
     // groups of rows for 1, 2 or 4 warps of a row group (a test per group cost 45 % at 32 rows)
     nt = M <= 16 ? 2 : M <= 24 ? 3 : M <= 32 ? 4 : M <= 48 ? 6 : M <= 64 ? 8 : M <= 96 ? 12 : 16;
   } else {
@@ -616,15 +643,8 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   if (!int8)
     return q4 ? few_launch_f16<FEW_Q4_F16>(ctx, nt, map, a)
               : few_launch_f16<FEW_Q8_F16>(ctx, nt, map, a);
-  switch (nt) {
-    case 2: return few_launch<FEW_Q8_INT8, 1, 2, 1, 1>(ctx, map, a, grid);
-    case 3: return few_launch<FEW_Q8_INT8, 1, 3, 1, 1>(ctx, map, a, grid);
-    case 4: return few_launch<FEW_Q8_INT8, 1, 4, 1, 1>(ctx, map, a, grid);
-    case 6: return few_launch<FEW_Q8_INT8, 1, 3, 2, 1>(ctx, map, a, grid);
-    case 8: return few_launch<FEW_Q8_INT8, 1, 4, 2, 1>(ctx, map, a, grid);
-    case 12: return few_launch<FEW_Q8_INT8, 1, 3, 4, 1>(ctx, map, a, grid);
-    default: return few_launch<FEW_Q8_INT8, 1, 4, 4, 1>(ctx, map, a, grid);
-  }
+  return tile == 112 ? few_launch_int8<112>(ctx, nt, map, a, grid)
+                     : few_launch_int8<128>(ctx, nt, map, a, grid);
 }
 
 }  // namespace kanso

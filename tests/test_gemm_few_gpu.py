@@ -93,9 +93,9 @@ def several_calls(ctx, kb, torch, fmt, blocks, x, N, act, calls=4):
     return [y.cpu().numpy() for y in ys]
 
 
-# Matrices whose K stays whole: 93 tiles of 112 rows, and a K of fewer than four units
+# Matrices whose K stays whole: 93 tiles of 112 rows, 148 of 128, and a K of fewer than four units
 @pytest.mark.parametrize("M,N,K", [(24, 10400, 2048), (48, 10400, 2048), (64, 10400, 2048),
-                                   (96, 10400, 2048),
+                                   (96, 10400, 2048), (33, 18944, 2304), (128, 18944, 2304),
                                    (16, 1000, 512), (128, 300, 768), (9, 131, 256)])
 def test_q8_activations_bit_exact(ctx, kb, oracle, torch_cuda, M, N, K):
     blocks = matrix("q8_0", N, K)
