@@ -5,9 +5,9 @@
 //   y[M,N] = x[M,K] @ W[N,K]^T,  W in GGUF Q8_0 / Q4_K blocks, x and y f32.
 //
 // This is the three-product form used by the decode step's chain of matmuls (more than 8
-// sequences) and by shapes whose rows do not start on 16-byte boundaries; single matmuls of 9..512
-// rows with aligned rows take the TMA-staged kernel in gemm_tma.cu, KANSO_ACT_Q8 batches the
-// weight-streaming kernel in gemm_few.cu.
+// sequences) and by shapes whose rows do not start on 16-byte boundaries; single matmuls with
+// aligned rows take the weight-streaming kernel in gemm_few.cu (few activation rows, KANSO_ACT_Q8) or the
+// TMA-staged one in gemm_tma.cu.
 //
 // Mapping. The weight matrix is the 128-row operand of the MMA (A, K-major) and the
 // activations are the narrow operand (B, K-major, 16..128 rows), so one CTA owns 128 weight

@@ -23,15 +23,23 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
 
 int32_t matmul_dispatch(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const float* x,
                         float* y, int64_t M, int64_t N, int64_t K, int32_t act_mode) {
-  // 9..64 activation rows (Q8_0: from two rows on), and any number above 8 with Q8 activations: the
-  // weight-streaming kernel, in passes of at most 64 (128) rows. Against the kernels below, which
-  // keep what it does not take, us per product with weights from memory (14336 x 4096): Q8_0 at
-  // 2 / 24 / 64 rows 22 / 29 / 50 against 42 / 46 / 50; Q4_K at 16 / 24 / 64 rows 26 / 30 / 50
-  // against 46 / 48 / 54. Fewer Q4_K rows keep the int8 GEMV's finer activations. Q8 activations
-  // at 16 / 32 / 64 / 128 rows: 27 / 38 / 61 / 100 against the 127 / 128 / 129 / 168 of a tcgen05
-  // kind::i8 form that drained an accumulator per block.
-  const bool few = act_mode == KANSO_ACT_Q8 ? M > 8 && dtype == KANSO_DTYPE_Q8_0
-                                            : M <= 64 && M >= (dtype == KANSO_DTYPE_Q8_0 ? 2 : 9);
+  // 9..48 activation rows (Q8_0: from two rows on), mostly 49..64 too, and any number above 8 with Q8
+  // activations: the weight-streaming kernel, in passes of at most 64 (128) rows. us per product, all
+  // in graphs of products behind one another over more than 300 MB of weights, against the kernels
+  // below, which keep what it does not take. 14336 x 4096: Q8_0 at 2 / 24 / 48 / 64 rows 16 / 20 / 27 /
+  // 34 against 30 / 32 / 33 / 34, Q4_K at 16 / 24 / 48 / 64 rows 17 / 20 / 28 / 33 against 31 / 33 / 34 /
+  // 36; 4096 x 4096 Q8_0 at 9 / 32 / 48 rows 8 / 12 / 13 against 12 / 15 / 15. Fewer Q4_K rows keep the
+  // int8 GEMV's finer activations. Q8 activations at 16 / 32 / 64 / 128 rows: 20 / 27 / 41 / 68 against
+  // the 87 / 87 / 87 / 113 of a tcgen05 kind::i8 form that drained an accumulator per block.
+  // 49..64 rows take one CTA per SM with all its registers: between one and nine units for it (128
+  // weight rows x 256 k) they do not share out evenly, and the kernel below is the faster one: Q8_0
+  // at 64 rows of 4096 x 4096 17.6 against 15.3, 8192 x 4096 23.6 and 22.4; but 2048 x 1024 7.5 and
+  // 10.2, 4096 x 14336 35 and 38, 11008 x 4096 29 and 36.
+  const int64_t units = (N + 127) / 128 * (K / 256);
+  const bool even = !ctx || units <= ctx->sm_count || units >= 9 * (int64_t)ctx->sm_count;
+  const bool few = act_mode == KANSO_ACT_Q8
+                       ? M > 8 && dtype == KANSO_DTYPE_Q8_0
+                       : M <= (even ? 64 : 48) && M >= (dtype == KANSO_DTYPE_Q8_0 ? 2 : 9);
   if (few && w && x && y) {
     bool all = true;
     for (int64_t m0 = 0; m0 < M && all;) {
@@ -48,7 +56,7 @@ int32_t matmul_dispatch(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const
   // More rows on a matrix whose rows start on 16-byte boundaries: the TMA-staged tcgen05 GEMM, up
   // to 512 rows per pass over the weights (96 rows of 14336 x 4096: 57 against 68 us of the
   // weight-streaming kernel, whose mma.sync rate is the bound there).
-  const bool tma_rows = M > 64;
+  const bool tma_rows = M > 64 || (M > 48 && !even);
   if (tma_rows && act_mode == KANSO_ACT_F32 && N > 0 && K > 0 && w && x && y) {
     bool all = true;
     for (int64_t m0 = 0; m0 < M && all; m0 += 512) {
