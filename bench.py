@@ -570,12 +570,11 @@ def prefill_attention_leg(torch, kb, O, ctx, stream):
     e1.record(stream)
     torch.cuda.synchronize()
     us = e0.elapsed_time(e1) * 1e3 / (iters * layers)
-    # every query row walks its causal prefix: the records one launch touches, counted per row
+    # every query row sees its causal prefix
     row_tokens = sum(int(c) - chunk + i + 1 for c in ctx_lens for i in range(chunk))
     flops = 4.0 * row_tokens * H * hd  # QK and PV
     res = {"check_vs_oracle_rel_err": err, "sequences": S, "chunk": chunk, "cached": cached,
            "us_per_launch": us, "query_rows_per_s": T / us * 1e6,
-           "cache_GB/s_per_row_walk": row_tokens * KH * (2 * hd + 8) / us / 1e3,
            "GFLOP/s": flops / us / 1e3}
     pool.destroy()
     return res

@@ -147,7 +147,10 @@ int32_t kanso_cuda_gemv_q4_k(kanso_cuda_ctx* ctx, const void* w, const float* x,
 
 /* LinearWeight::forward, y[M,N] = x[M,K] @ W[N,K]^T — src/weights.rs:43-45,
  * callers src/model.rs:390-397. x f32[M,K] row-major, y f32[M,N] row-major.
- * act_mode is KANSO_ACT_F32 or KANSO_ACT_Q8 (Q4_K accepts KANSO_ACT_F32 only). */
+ * act_mode is KANSO_ACT_F32 or KANSO_ACT_Q8 (Q4_K accepts KANSO_ACT_F32 only).
+ * Products of 2..64 rows (Q4_K: 9..64), and larger ones on matrices of at most 5888 rows, add parts of
+ * K in no fixed order: repeated calls may differ in the last bits. KANSO_ACT_Q8 with more than eight rows
+ * equals the CPU statement bit for bit where N > 10304 or K < 1024 (148 SMs), K % 256 == 0. */
 int32_t kanso_cuda_gemm_q8_0(kanso_cuda_ctx* ctx, const void* w, const float* x, float* y,
                              int64_t M, int64_t N, int64_t K, int32_t act_mode);
 int32_t kanso_cuda_gemm_q4_k(kanso_cuda_ctx* ctx, const void* w, const float* x, float* y,

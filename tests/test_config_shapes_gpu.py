@@ -60,10 +60,10 @@ def test_batched_matmul_at_config_shapes(ctx, kb, oracle, torch_cuda, fmt, N, M)
 
 
 @pytest.mark.parametrize("M", [2, 3, 5, 7])
-def test_q8_0_few_rows_take_the_tensor_core_gemm(ctx, kb, oracle, torch_cuda, M):
-    """Q8_0 matrices whose rows start on 16-byte boundaries go to the TMA-staged GEMM from two
-    activation rows on (below nine rows the int8-MMA GEMV used to take them): same bound, and the
-    rows beyond M of the 16-row accumulator tile must not leak into y."""
+def test_q8_0_few_rows_stay_inside_y(ctx, kb, oracle, torch_cuda, M):
+    """Q8_0 matrices whose rows start on 16-byte boundaries go to the weight-streaming GEMM
+    (csrc/gemm_few.cu) from two activation rows on: same bound, and the rows beyond M of its groups of
+    eight must not leak into y."""
     torch = torch_cuda
     N = 4096
     rows2d, W = quantized(oracle, kb, ctx, "q8_0", N)
@@ -104,10 +104,10 @@ def test_q8_activation_mode_at_config_shapes(ctx, kb, oracle, torch_cuda, M):
 
 @pytest.mark.parametrize("M", [16, 100, 128])
 def test_q8_activation_gemm_is_bit_exact_when_k_is_not_split(ctx, kb, oracle, torch_cuda, M):
-    """More than 8 rows in KANSO_ACT_Q8 mode run on tcgen05 kind::i8: the int32 block sums are
-    exact and the f32 scaling and additions follow scalar_dot_q8_0_q8_0 / scalar_gemv_q8_0
+    """More than 8 rows in KANSO_ACT_Q8 mode run on int8 mma.sync (csrc/gemm_few.cu): the int32 block
+    sums are exact and the f32 scaling and additions follow scalar_dot_q8_0_q8_0 / scalar_gemv_q8_0
     (src/quant/q8_0.rs:60-66,82-92) operation for operation, so on a matrix wide enough not to be
-    split along K (14336 rows = 112 CTAs) the result equals the oracle's bit for bit."""
+    split along K (14336 rows = 128 tiles) the result equals the oracle's bit for bit."""
     torch = torch_cuda
     N = 14336
     rows2d, W = quantized(oracle, kb, ctx, "q8_0", N)
