@@ -1,5 +1,6 @@
 """GPU: products of a few activation rows (csrc/gemm_few.cu) against the oracle, at the edges of its
-tiles: 128 weight rows, 8 activation rows, units of 256 k dealt out in runs that cross tiles.
+tiles: 128 weight rows (int8: 112 or 128), 8 activation rows, units of 256 k, one a CTA and in runs that
+cross tiles.
 
 Tolerances: both f16 operands are rounded once, 2^-11 of each value, so the error of a sum of K products of
 independent sign is about 2^-11 of its root mean square (max over the results: 1e-3 of the largest
@@ -93,6 +94,25 @@ def several_calls(ctx, kb, torch, fmt, blocks, x, N, act, calls=4):
     return [y.cpu().numpy() for y in ys]
 
 
+# 1456 units of 112 tiles over 148 or 296 CTAs: runs longer than the ring that begin and end inside
+# tiles; 33 x 16 units: one to four a CTA; 2 x 16: sixteen CTAs to a tile
+@pytest.mark.parametrize("N,K", [(14336, 3328), (4099, 4096), (200, 4096)])
+@pytest.mark.parametrize("fmt,M", [("q8_0", m) for m in (2, 9, 17, 32, 48, 64)] +
+                         [("q4_k", m) for m in (9, 24, 25, 48, 64)])
+def test_runs_across_tiles(ctx, kb, oracle, torch_cuda, fmt, M, N, K):
+    """Long runs give the oracle's results. Calls differ by the order in which a tile's runs are added:
+    up to 16 additions of 2^-24 of the sums each, 1e-6 of the largest result."""
+    blocks = matrix(fmt, N, K)
+    x = data(M, 1, K)[1]
+    got = several_calls(ctx, kb, torch_cuda, fmt, blocks, x, N, kb.ACT_F32)
+    pick = some_rows(N)
+    sub = np.ascontiguousarray(blocks[pick]).reshape(-1)
+    ref = (oracle.gemm_q8_0 if fmt == "q8_0" else oracle.gemm_q4_k)(sub, x, M, pick.size, K)
+    for y in got:
+        assert rel_err(y[:, pick], ref) <= 1e-3
+        assert rel_err(y, got[0]) <= 1e-6
+
+
 # Matrices whose K stays whole: 93 tiles of 112 rows, 148 of 128, and a K of fewer than four units
 @pytest.mark.parametrize("M,N,K", [(24, 10400, 2048), (48, 10400, 2048), (64, 10400, 2048),
                                    (96, 10400, 2048), (33, 18944, 2304), (128, 18944, 2304),
@@ -113,3 +133,17 @@ def test_q8_activations_halved_k_repeats(ctx, kb, oracle, torch_cuda, M, N, K):
     got = several_calls(ctx, kb, torch_cuda, "q8_0", blocks, data(M, 1, K)[1], N, kb.ACT_Q8)
     for again in got[1:]:
         assert (got[0] == again).all()
+
+
+@pytest.mark.parametrize("M", [513, 530, 576, 584])
+@pytest.mark.parametrize("fmt", ["q8_0", "q4_k"])
+def test_rows_behind_a_pass_of_512(ctx, kb, oracle, torch_cuda, fmt, M):
+    N, K = 300, 512
+    w, x = data(M, N, K)
+    if fmt == "q8_0":
+        blocks, dt = oracle.quantize_weights_q8_0(w), kb.DTYPE_Q8_0
+        ref = oracle.gemm_q8_0(blocks, x, M, N, K)
+    else:
+        blocks, dt = oracle.quantize_weights_q4_k(w), kb.DTYPE_Q4_K
+        ref = oracle.gemm_q4_k(blocks, x, M, N, K)
+    assert rel_err(run(ctx, kb, torch_cuda, dt, blocks, x, N, kb.ACT_F32), ref) <= 1e-3
