@@ -340,6 +340,18 @@ __device__ __forceinline__ void tc_dequant_q4_k(const uint8_t* raw_stage, int s,
   }
 }
 
+// The producers' barrier: true for all of them when one of them has seen the CTA give up.
+__device__ __forceinline__ bool producers_abort(bool mine) {
+  uint32_t any;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred.aligned q, 1, %2, p;\n"
+      "selp.b32 %0, 1, 0, q;\n}\n"
+      : "=r"(any)
+      : "r"((uint32_t)mine), "n"(TC_PRODUCERS)
+      : "memory");
+  return any != 0;
+}
+
 // Warps 0-15 produce the A tiles (raw-byte copies, dequantisation) and run the epilogue; warp 16
 // fetches the B tiles with one bulk copy per stage and issues the MMAs, so building descriptors
 // and issuing never delays the next stage's dequantisation. Buffer indices and mbarrier
@@ -412,14 +424,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     uint32_t reuse_par = 1;  // parity of done[buf] for the previous use of the buffer
     for (int s = s0; s < s1; ++s) {
       const int it = s - s0;
-      copy_raw(s + 3, (it + 3) & (TC_RAW_DEPTH - 1));
       // the A buffer of this stage was last read by the MMAs of stage s - NS
       if (it >= NS && !mbar_wait_bounded(&done[buf], reuse_par)) *abort_flag = 1;
-      // all but the three newest groups have landed: raw(s) is in shared memory
-      asm volatile("cp.async.wait_group 3;" ::: "memory");
-      // producers' barrier: every producer's copies of this stage are visible to all
-      asm volatile("bar.sync 1, %0;" ::"n"(TC_PRODUCERS) : "memory");
-      if (*abort_flag) break;
+      // all but the two newest groups have landed: raw(s) is in shared memory
+      asm volatile("cp.async.wait_group 2;" ::: "memory");
+      // producers' barrier: every producer's copies of this stage are visible to all, and all have read
+      // the raw bytes of the stage before, whose slot is filled again only now. They leave together.
+      if (producers_abort(*abort_flag != 0)) break;
+      copy_raw(s + 3, (it + 3) & (TC_RAW_DEPTH - 1));
       uint8_t* Ab = As + buf * TC_A_STAGE;
       const uint8_t* rs = Raw + (it & (TC_RAW_DEPTH - 1)) * TC_RAW_STAGE;
       if (FMT == TC_FMT_Q8_0)
