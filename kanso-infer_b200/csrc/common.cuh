@@ -77,6 +77,16 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
       : "memory");
 }
 
+// One thread of a converged warp, chosen by the hardware. Threads that issue tcgen05 or bulk-copy
+// instructions are chosen this way: their operands live in uniform registers, and behind a test of the
+// lane number the compiler cannot know that one thread alone is active.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+
 // Programmatic dependent launch: let the next kernel of the stream start launching, and wait
 // until the kernel before this one has completed and its writes are visible. Both are no-ops
 // for a launch without the attribute.

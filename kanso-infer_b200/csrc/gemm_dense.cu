@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(GD_THREADS)
   const int k1 = min(k0 + a.steps_per_split, a.k_steps);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int k = k0, i = 0; k < k1; ++k, ++i) {
         const int s = i % S::kStages;
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(GD_THREADS)
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_n = NT;
       const uint32_t idesc = tc_idesc_bf16(128, idesc_n);
       bool ok = true;

@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(TILE / (16 * RT) * OTHER * 32 + 32, CTAS)
   pdl_launch_dependents();
 
   if (warp == WARPS) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto weights = [&](int u, int slot) {
         mbar_arrive_expect_tx(&full[slot], STAGE);
         tma_load_2d(smem + slot * STAGE, &tmap, u % a.chunks * (few_row_bytes<FORM>() / 4),

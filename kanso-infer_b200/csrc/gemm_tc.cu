@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else if (warp == TC_PRODUCERS / 32 + 2) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---- B tiles (packed activations) by bulk copy, one stage per shared-memory buffer; a
       // buffer is refilled once the MMAs of the stage that used it last have retired
       const uint8_t* bsrc = reinterpret_cast<const uint8_t*>(a.xp);
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     // ---- MMA issuers: thread `me` owns the stages it = me, me + 2, ... and the accumulator
     // columns [me * acc_cols, me * acc_cols + Mt); the two never read the same tile at once
     const int me = warp - TC_PRODUCERS / 32;
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = tc_idesc_f16(TC_TILE_N, a.Mt);
       const uint32_t a_k = (2 * (TC_TILE_N * 16)) >> 4, b_k = (2 * (a.Mt * 16)) >> 4;  // per 16 k
       const uint32_t acc = tmem_base + (uint32_t)me * acc_cols;

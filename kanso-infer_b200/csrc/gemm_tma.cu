@@ -99,10 +99,12 @@ int32_t tma_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   while (tiles_n * ksplit * 2 <= ctx->sm_count + ctx->sm_count / 4 &&
          boxes_total / (ksplit * 2) >= 4)
     ksplit *= 2;
-  // activation units per ring slot: a whole stage (8 k-steps) when that stays at or below
-  // 16 KB, else the largest power-of-two share of it that does
+  // activation units per ring slot: a whole stage (8 k-steps) when a slot holds that, else the
+  // largest power-of-two share of it that fits
+  const int b_slots = Mt <= 128 ? TM_B_SLOTS_TWO : TM_B_SLOTS_ONE;
+  const int b_slot = Mt <= 128 ? TM_B_SLOT_TWO : TM_B_SLOT_ONE;
   int ub = 1;
-  while (ub * 2 <= 8 && ub * 2 * 32 * Mt <= 16384) ub *= 2;
+  while (ub * 2 <= 8 && ub * 2 * 32 * Mt <= b_slot) ub *= 2;
 
   CUtensorMap tmap;
   const cuuint64_t gdim[2] = {(cuuint64_t)row_bytes, (cuuint64_t)N};
@@ -154,7 +156,7 @@ int32_t tma_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   a.ub = ub;
   a.status = ctx->dev_status;
   const size_t smem = (size_t)TM_RAW_SLOTS * TM_BOX + (size_t)TM_A_STAGES * TM_A_STAGE +
-                      (size_t)TM_B_SLOTS * ub * 32 * Mt + 256;
+                      (size_t)b_slots * ub * 32 * Mt + 256;
   if (smem > (size_t)ctx->smem_optin)
     return fail(ctx, KANSO_ERR_UNSUPPORTED, "gemm_tma: %zu bytes of shared memory needed", smem);
   const dim3 grid(tiles_n, ksplit);

@@ -20,10 +20,16 @@ constexpr int TM_THREADS = 768;  // 24 warps: scheduler 0 holds the MMA issuer a
 constexpr int TM_TILE_N = 128;                 // weight rows per CTA = MMA M
 constexpr int TM_BOX_W = 128;                  // bytes of a weight row per box (the swizzle span)
 constexpr int TM_BOX = TM_TILE_N * TM_BOX_W;   // 16 KB per ring slot
-constexpr int TM_RAW_SLOTS = 5;  // measured: 4..7 slots and 2 or 3 A stages all within 3 %
+constexpr int TM_RAW_SLOTS = 4;  // measured: 3..7 slots and 2 or 3 A stages all within 3 %
 constexpr int TM_A_STAGES = 2;
 constexpr int TM_A_STAGE = 32768;  // 16 k-chunks of 8 positions x 128 rows x 16 bytes
-constexpr int TM_B_SLOTS = 4;
+// Activation ring: four slots of up to 16 KB for the two issuing threads of up to 128 rows, three of up
+// to 32 KB for the one of more rows. That thread pays about 500 cycles a slot for the wait, the fence and
+// the commit, whatever the slot holds: 512 rows of 14336 x 4096 in slots of one k-step 79 us, of
+// two 71 us; 256 rows in slots of two and of four 47 and 41 us.
+constexpr int TM_B_SLOTS_TWO = 4, TM_B_SLOT_TWO = 16384;
+constexpr int TM_B_SLOTS_ONE = 3, TM_B_SLOT_ONE = 32768;
+constexpr int TM_B_SLOTS_MAX = 4;
 constexpr int TM_FMT_Q8_0 = 0;
 constexpr int TM_FMT_Q4_K = 1;
 constexpr int TM_MAX_M = 512;
@@ -39,7 +45,7 @@ struct TmArgs {
   int row_bytes;       // bytes of one weight row
   int boxes_total;     // ceil(row_bytes / 128)
   int ksplit;          // CTAs along the stream; > 1: partial sums are added into y with atomics
-  int ub;              // activation units per ring slot (1, 2, 4 or 8)
+  int ub;              // activation units per ring slot (2, 4 or 8)
   int* status;
 };
 
@@ -264,13 +270,14 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
   uint8_t* Raw = smem;
   uint8_t* As = Raw + TM_RAW_SLOTS * TM_BOX;
   uint8_t* Bs = As + TM_A_STAGES * TM_A_STAGE;
-  uint64_t* raw_full = reinterpret_cast<uint64_t*>(Bs + TM_B_SLOTS * bslot_bytes);
+  const uint32_t b_slots = a.Mt <= 128 ? TM_B_SLOTS_TWO : TM_B_SLOTS_ONE;
+  uint64_t* raw_full = reinterpret_cast<uint64_t*>(Bs + b_slots * bslot_bytes);
   uint64_t* raw_empty = raw_full + TM_RAW_SLOTS;
   uint64_t* a_full = raw_empty + TM_RAW_SLOTS;
   uint64_t* a_empty = a_full + TM_A_STAGES;
   uint64_t* b_full = a_empty + TM_A_STAGES;
-  uint64_t* b_empty = b_full + TM_B_SLOTS;
-  uint64_t* acc_full = b_empty + TM_B_SLOTS;
+  uint64_t* b_empty = b_full + TM_B_SLOTS_MAX;
+  uint64_t* acc_full = b_empty + TM_B_SLOTS_MAX;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* issued_any = abort_flag + 1;  // [2]: did issuer i accumulate anything
@@ -302,7 +309,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
       mbar_init(&a_full[i], TM_PRODUCERS / 32);
       mbar_init(&a_empty[i], 1);
     }
-    for (int i = 0; i < TM_B_SLOTS; ++i) {
+    for (int i = 0; i < TM_B_SLOTS_MAX; ++i) {
       mbar_init(&b_full[i], 1);
       mbar_init(&b_empty[i], 1);
     }
@@ -399,7 +406,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
     // descriptor a constant offset from the stage's first. Issuer i owns the stages j = i,
     // i + nissue, ...: A buffer j % 2 and the TMEM columns [i * acc_cols, i * acc_cols + Mt).
     const int me = warp == 20 ? 1 : 0;
-    if (lane == 0 && me < nissue) {
+    if (me < nissue && elect_one()) {
       const bool two = a.Mt > 256;  // a second chunk of columns 256.. (single issuer only)
       const uint32_t idesc0 = tc_idesc_f16(TM_TILE_N, two ? 256 : a.Mt);
       const uint32_t idesc1 = tc_idesc_f16(TM_TILE_N, two ? a.Mt - 256 : 16);
@@ -421,7 +428,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
         const uint32_t l0 = (uint32_t)j * sps;  // first activation slot group of the stage
         // the activations of a stage arrive long before its weights are dequantised: their
         // barrier is looked at first, so that one fence covers both waits
-        if (!mbar_wait_bounded(&b_full[l0 % TM_B_SLOTS], (l0 / TM_B_SLOTS) & 1u)) ok = false;
+        if (!mbar_wait_bounded(&b_full[l0 % b_slots], (l0 / b_slots) & 1u)) ok = false;
         if (!mbar_wait_bounded(&a_full[abuf], a_par)) {
           ok = false;
           break;
@@ -434,13 +441,14 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
         const uint32_t hdr = FMT == TM_FMT_Q4_K ? (cm == 0u ? 0u : 9u - cm) : 99u;
         const uint32_t nvalid = o0 >= row_bytes ? 0u : min((uint32_t)CH, (row_bytes - o0 + 15u) >> 4);
         const uint32_t alo = adesc_lo0 + abuf * (TM_A_STAGE >> 4);
-        auto run = [&](auto ub_tag) {
+        auto run = [&](auto ub_tag, auto slots_tag) {
           constexpr int UB = decltype(ub_tag)::value;
+          constexpr uint32_t SLOTS = decltype(slots_tag)::value;
 #pragma unroll
           for (int g = 0; g < CH * UPC / UB; ++g) {
-            const uint32_t l = l0 + (uint32_t)g, bslot = l % TM_B_SLOTS;
+            const uint32_t l = l0 + (uint32_t)g, bslot = l % SLOTS;
             if (g > 0) {
-              if (!mbar_wait_bounded(&b_full[bslot], (l / TM_B_SLOTS) & 1u)) ok = false;
+              if (!mbar_wait_bounded(&b_full[bslot], (l / SLOTS) & 1u)) ok = false;
               tc_fence_after();
             }
             uint32_t blo = bdesc_lo0 + bslot * b_slot;
@@ -453,7 +461,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
                 const uint64_t ad = tc_desc_join(alo + (uint32_t)ks * a_kstep, adesc_hi);
                 const uint64_t bd = tc_desc_join(blo, bdesc_hi);
                 tc_mma_f16(acc_tmem, ad, bd, idesc0, acc);
-                if (UB == 1 && two)
+                if (UB == 2 && two)
                   tc_mma_f16(acc_tmem + 256u, ad, tc_desc_join(blo + 256u, bdesc_hi), idesc1, acc);
                 acc = 1;
               }
@@ -462,14 +470,15 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
             tc_commit(&b_empty[bslot]);
           }
         };
+        using std::integral_constant;
         if (ub == 8u)
-          run(std::integral_constant<int, 8>{});
-        else if (ub == 4u)
-          run(std::integral_constant<int, 4>{});
+          run(integral_constant<int, 8>{}, integral_constant<int, TM_B_SLOTS_TWO>{});
         else if (ub == 2u)
-          run(std::integral_constant<int, 2>{});
+          run(integral_constant<int, 2>{}, integral_constant<int, TM_B_SLOTS_ONE>{});
+        else if (nissue == 2)
+          run(integral_constant<int, 4>{}, integral_constant<int, TM_B_SLOTS_TWO>{});
         else
-          run(std::integral_constant<int, 1>{});
+          run(integral_constant<int, 4>{}, integral_constant<int, TM_B_SLOTS_ONE>{});
         tc_commit(&a_empty[abuf]);
       }
       issued_any[me] = acc;
@@ -481,7 +490,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
     __syncwarp();
   } else if (warp == TM_PRODUCERS / 32 + 1) {
     // ---- weight loader: one box per ring slot, as far ahead as the ring allows ----
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int box = first, idx = 0; box < b1; ++box, ++idx) {
         const int slot = idx % TM_RAW_SLOTS;
@@ -501,14 +510,14 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
     __syncwarp();
   } else if (warp == TM_PRODUCERS / 32 + 2) {
     // ---- activation loader: ring slots of `ub` units, contiguous in the packed buffer ----
-    if (lane == 0) {
+    if (elect_one()) {
       pdl_wait();  // the pack kernel has written the activations
       const uint32_t g0 = (uint32_t)b0 * 8u * UPC / (uint32_t)a.ub;
       const uint32_t g1 = (uint32_t)b1 * 8u * UPC / (uint32_t)a.ub;
       uint32_t issued = 0;
       for (uint32_t g = g0; g < g1; ++g) {
-        const uint32_t l = g - g0, slot = l % TM_B_SLOTS;
-        if (!tm_wait_polite(&b_empty[slot], ((l / TM_B_SLOTS) & 1u) ^ 1u) || *abort_flag) {
+        const uint32_t l = g - g0, slot = l % b_slots;
+        if (!tm_wait_polite(&b_empty[slot], ((l / b_slots) & 1u) ^ 1u) || *abort_flag) {
           *abort_flag = 1;
           break;
         }
@@ -517,8 +526,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
                  &b_full[slot]);
         issued = l + 1;
       }
-      for (uint32_t l = issued > TM_B_SLOTS ? issued - TM_B_SLOTS : 0; l < issued; ++l)
-        tm_wait_polite(&b_full[l % TM_B_SLOTS], (l / TM_B_SLOTS) & 1u);
+      for (uint32_t l = issued > b_slots ? issued - b_slots : 0; l < issued; ++l)
+        tm_wait_polite(&b_full[l % b_slots], (l / b_slots) & 1u);
     }
     __syncwarp();
   }

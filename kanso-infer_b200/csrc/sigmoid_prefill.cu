@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
     __syncwarp();
   } else if (warp == 9) {
     // ---- products ----
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t id_s = tc_idesc_bf16(SP_Q, SP_K);
       const uint32_t id_o = tc_idesc_bf16(SP_Q, p.nv) | (1u << 16);  // B is N-major
       bool ok = mbar_wait_abort(&q_full, 0, &abort_flag);

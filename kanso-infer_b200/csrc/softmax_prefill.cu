@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1)
 
   if (warp == 8 || warp == 10) {
     // ---- copies ----
-    if (lane == 0) {
+    if (elect_one()) {
       const bool keys = warp == 8;
       const int stages = keys ? p.k_stages : p.v_stages;
       const uint32_t bytes = keys ? k_bytes : v_bytes;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1)
     __syncwarp();
   } else if (warp == 9) {
     // ---- scores ----
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = tc_idesc_bf16(SX_Q, SX_K);
       const uint32_t queries = smem_u32(Qs), keys = smem_u32(Ks);
       bool ok = mbar_wait_abort(&q_full, 0, &abort_flag);
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1)
     __syncwarp();
   } else if (warp == 11) {
     // ---- weights x values ----
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = tc_idesc_bf16(SX_Q, p.nv) | (1u << 16);  // B is N-major
       const uint64_t weights = tc_smem_desc_sw128(smem_u32(Ps));
       const uint64_t values = tc_smem_desc_nmajor(smem_u32(Vs), SX_K * 128u);
