@@ -41,32 +41,88 @@
 
 namespace kanso {
 
-template <int FMT>
-__global__ void tm_pack_kernel(const float* __restrict__ x, __half* __restrict__ bp, int M, int Mt,
-                               int K, int units_total, const TmZero zero) {
+// Activations into stream order. A tile is 32 rows x 256 k (K % 256 == 0 for both formats here: rows of
+// blocks that start on 16 bytes), which is 17 chunks of a Q8_0 stream and 36 half k-steps of a Q4_K one:
+// it is read along k, whole sectors, rounded to f16 in shared memory and written with lanes along the
+// rows, 512 bytes at a time. A thread that gathered its 8 values from memory itself, its neighbours a row
+// apart, took 17 us for 512 x 4096 and 31 us for 512 x 14336 (8.4 and 29 MB read, half of that written).
+// Tiles behind the last k are the stream's padding: zeros.
+constexpr int PACK_ROWS = 32, PACK_K = 256;
+constexpr int PACK_PITCH = PACK_K + 2;  // an odd number of words: lanes along the rows, 32 banks
+template <int FMT, bool VEC>
+__global__ void __launch_bounds__(256)
+    tm_pack_kernel(const float* __restrict__ x, __half* __restrict__ bp, int M, int Mt, int K,
+                   int units_total, const TmZero zero) {
+  // unit halves (8 positions of every row) of a tile
+  constexpr int HALVES = FMT == TM_FMT_Q8_0 ? 2 * (PACK_K / 32 * Q8_BYTES / 16)
+                                            : 4 * (Q4K_BYTES / 16);
+  __shared__ __half tile[PACK_ROWS * PACK_PITCH];
   pdl_launch_dependents();
   pdl_wait();  // x (and the readers of the buffer cleared here) belong to earlier kernels
-  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t j = gtid; j < zero.n; j += nthreads) zero.p[j] = 0.f;
-  const int64_t total = (int64_t)units_total * 2 * Mt;
-  for (int64_t i = gtid; i < total; i += nthreads) {
-    const int m = (int)(i % Mt);
-    const int uk = (int)(i / Mt);  // unit * 2 + k-chunk
-    const int u = uk >> 1, kc8 = uk & 1;
-    __align__(16) __half v[8];
+  const int64_t cta = blockIdx.y * (int64_t)gridDim.x + blockIdx.x;
+  const int64_t nthreads = (int64_t)gridDim.x * gridDim.y * blockDim.x;
+  for (int64_t j = cta * blockDim.x + threadIdx.x; j < zero.n; j += nthreads) zero.p[j] = 0.f;
+  const int k0 = blockIdx.x * PACK_K, m0 = blockIdx.y * PACK_ROWS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (k0 < K) {
+    // warp: rows warp, warp + 8, ...; lane: four values at 4 * lane and 128 further on
+    float4 v[PACK_ROWS / 8][2];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      int k;
-      if (FMT == TM_FMT_Q8_0)
-        k = tm_k_of_q8_0(u, 8 * kc8 + e);
-      else
-        k = tm_k_of_q4_k(u >> 1, u & 1, 8 * kc8 + e);
-      const float f = (m < M && k >= 0 && k < K) ? x[(int64_t)m * K + k] : 0.f;
-      v[e] = __float2half_rn(f);
-    }
-    *reinterpret_cast<uint4*>(bp + i * 8) = *reinterpret_cast<const uint4*>(v);
+    for (int i = 0; i < PACK_ROWS / 8; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = m0 + warp + 8 * i;
+        const float* src = x + (int64_t)m * K + k0 + h * 128 + lane * 4;
+        v[i][h] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m < M) {
+          if (VEC)
+            v[i][h] = *reinterpret_cast<const float4*>(src);
+          else
+            v[i][h] = make_float4(src[0], src[1], src[2], src[3]);
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < PACK_ROWS / 8; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        __half2* dst = reinterpret_cast<__half2*>(tile + (warp + 8 * i) * PACK_PITCH + h * 128 +
+                                                  lane * 4);
+        dst[0] = __floats2half2_rn(v[i][h].x, v[i][h].y);
+        dst[1] = __floats2half2_rn(v[i][h].z, v[i][h].w);
+      }
+    __syncthreads();
   }
+  const int m = m0 + lane;
+  const int first = blockIdx.x * HALVES;
+  const uint16_t* row = reinterpret_cast<const uint16_t*>(tile) + lane * PACK_PITCH;
+  for (int j = warp; j < HALVES && first + j < 2 * units_total; j += 8) {
+    uint32_t o[4] = {};
+    if (k0 < K) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int k = FMT == TM_FMT_Q8_0 ? tm_k_of_q8_0(j >> 1, 8 * (j & 1) + e)
+                                         : tm_k_of_q4_k(j >> 2, (j >> 1) & 1, 8 * (j & 1) + e);
+        if (k >= 0) o[e >> 1] |= (uint32_t)row[k] << (16 * (e & 1));
+      }
+    }
+    if (m < Mt)
+      *reinterpret_cast<uint4*>(bp + ((int64_t)(first + j) * Mt + m) * 8) =
+          make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+template <int FMT>
+static int32_t tm_pack(kanso_cuda_ctx* ctx, const float* x, void* bp, int M, int Mt, int K,
+                       int units_total, const TmZero& zero) {
+  constexpr int UNITS = FMT == TM_FMT_Q8_0 ? PACK_K / 32 * Q8_BYTES / 16 : 2 * (Q4K_BYTES / 16);
+  const dim3 grid((unsigned)((units_total + UNITS - 1) / UNITS),
+                  (unsigned)((Mt + PACK_ROWS - 1) / PACK_ROWS));
+  auto kern = aligned16(x) ? tm_pack_kernel<FMT, true> : tm_pack_kernel<FMT, false>;
+  const cudaError_t le = launch_dependent(ctx, kern, grid, dim3(256), 0, x,
+                                          reinterpret_cast<__half*>(bp), M, Mt, K, units_total,
+                                          zero);
+  if (le != cudaSuccess) return cuda_fail(ctx, le, "gemm_tma pack launch");
+  return after_launch(ctx, "gemm_tma pack activations");
 }
 
 // y[M,N] = x[M,K] @ W^T for 9..512 activation rows (fewer than 49 are gemm_few.cu's, and come here
@@ -128,20 +184,10 @@ int32_t tma_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
     zero.p = y;
     zero.n = M * N;
   }
-  const int64_t pack_items = (int64_t)units_total * 2 * Mt;
-  int64_t pack_blocks = (pack_items + 255) / 256;
-  if (pack_blocks > 8 * ctx->sm_count) pack_blocks = 8 * ctx->sm_count;
-  cudaError_t le;
-  if (dtype == KANSO_DTYPE_Q8_0)
-    le = launch_dependent(ctx, tm_pack_kernel<TM_FMT_Q8_0>, dim3((unsigned)pack_blocks), dim3(256),
-                          0, x, reinterpret_cast<__half*>(scratch), (int)M, Mt, (int)K,
-                          units_total, zero);
-  else
-    le = launch_dependent(ctx, tm_pack_kernel<TM_FMT_Q4_K>, dim3((unsigned)pack_blocks), dim3(256),
-                          0, x, reinterpret_cast<__half*>(scratch), (int)M, Mt, (int)K,
-                          units_total, zero);
-  if (le != cudaSuccess) return cuda_fail(ctx, le, "gemm_tma pack launch");
-  int32_t st = after_launch(ctx, "gemm_tma pack activations");
+  const int32_t st =
+      dtype == KANSO_DTYPE_Q8_0
+          ? tm_pack<TM_FMT_Q8_0>(ctx, x, scratch, (int)M, Mt, (int)K, units_total, zero)
+          : tm_pack<TM_FMT_Q4_K>(ctx, x, scratch, (int)M, Mt, (int)K, units_total, zero);
   if (st) return st;
 
   TmArgs a;
