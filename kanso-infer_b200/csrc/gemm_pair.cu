@@ -7,7 +7,7 @@
 // For the experts' silu(gate) * up each CTA's 128 rows are 64 of the gate and the same 64 of the up matrix,
 // in lanes that lie 64 apart: the warps that store them exchange halves through shared memory. (Two
 // accumulators of 128 rows in each CTA fill TMEM, so that every tile waits for the stores of the one
-// before: 104 us where this form takes GU_US.)
+// before: 104 us where this form takes 74.)
 //
 // One pair of CTAs per two SMs stays for the whole product and takes tiles in turn. One thread copies
 // (tensor maps, 128-byte swizzle, K-major), one thread of the even CTA issues the products of both, and
@@ -36,6 +36,7 @@ constexpr int GP_BOX = 32;       // activation rows per copy where the tile's ro
 constexpr int GP_STAGE = 2 * GP_HALF;
 constexpr int GP_STAGES = 6;
 constexpr int GP_ACCS = 2;  // tiles whose results TMEM holds
+constexpr uint32_t GP_POLLS = 1u << 18;  // about a second: a poll that finds nothing lasts 4 us
 constexpr size_t GP_SMEM = (size_t)GP_STAGE * GP_STAGES + 1024;
 
 // What `tiles` of n activation rows cost `pairs` pairs, in cycles per 16 columns: a wave takes the products'
@@ -50,6 +51,7 @@ struct GpTiles {
   int row_tiles;   // of a group, where all are alike
   int n;           // activation rows of a tile, likewise
   int box;         // activation rows per copy
+  int most;        // tiles there can be at the most, whatever the offsets say
 };
 
 struct GpTile {
@@ -78,6 +80,7 @@ __device__ __forceinline__ int gp_max_n(const GemmDenseArgs& a, const GpTiles& t
 // Tile `tile`, by a whole warp; the same answer in both CTAs. false: past the last one.
 __device__ __forceinline__ bool gp_tile(const GemmDenseArgs& a, const GpTiles& t, int max_n, int tile,
                                         int lane, GpTile* out) {
+  if (tile >= t.most) return false;
   const int row_tile = tile / t.col_tiles;
   out->col = tile - row_tile * t.col_tiles;
   if (!a.offsets) {
@@ -126,8 +129,7 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
-                   : "memory");
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // The even CTA's copy of a barrier at the same place of its shared memory.
 __device__ __forceinline__ uint32_t even_bar(const uint64_t* bar) {
@@ -141,7 +143,7 @@ __device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
 // Waits are for arrivals of the other CTA too.
 __device__ __forceinline__ bool mbar_wait_pair(uint64_t* bar, uint32_t parity,
                                                volatile int* abort_flag) {
-  for (uint32_t i = 0; i < (1u << 22); ++i) {
+  for (uint32_t i = 0; i < GP_POLLS; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
@@ -193,7 +195,7 @@ __device__ __forceinline__ void pair_commit(uint64_t* bar) {
 __device__ __forceinline__ bool partners_any(int bar, bool mine) {
   uint32_t any;
   asm volatile(
-      "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred.aligned q, %2, 64, p;\n"
+      "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred q, %2, 64, p;\n"
       "selp.b32 %0, 1, 0, q;\n}\n"
       : "=r"(any)
       : "r"((uint32_t)mine), "r"(bar)
@@ -244,6 +246,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     mbar_fence_init();
     abort_flag = 0;
   }
+  cluster_sync();
+  pdl_launch_dependents();
+  pdl_wait();
+  // TMEM only once the kernels in front have ended: a CTA that waits for it waits without a limit
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                      smem_u32(&tmem_slot))
@@ -254,8 +260,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  pdl_launch_dependents();
-  pdl_wait();
   const int max_n = gp_max_n(a, tiles, lane, step);
 
   if (warp == 0) {
@@ -342,6 +346,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       const RowPlace place(a, t.group);
       for (int c = half * 16; c < t.n && c < t.valid; c += 32) {
         uint32_t r0[16];
+        __syncwarp();
         tmem_ld16(acc + c, r0);
         const int64_t row0 = t.first + c;
         const int valid = t.valid - c;
@@ -418,10 +423,11 @@ int32_t launch_gemm_pair(kanso_cuda_ctx* ctx, const DenseMat& w, const DenseMat*
   t.row_tiles = 1;
   t.n = 0;
   t.box = GP_BOX;
-  int64_t total;
+  int64_t total, most;
   if (r.offsets) {
     if (per < 96) return KANSO_OK;
     total = t.col_tiles * ((r.T + GP_MAX_N - 1) / GP_MAX_N);
+    most = t.col_tiles * (r.T / 128 + r.groups);  // gp_max_n: 128 and more
   } else {
     // equal parts of a group's rows: the number of them with which the last wave is fullest
     const int64_t cols = (int64_t)t.col_tiles * r.groups;
@@ -438,8 +444,10 @@ int32_t launch_gemm_pair(kanso_cuda_ctx* ctx, const DenseMat& w, const DenseMat*
     if (!best) return KANSO_OK;
     t.row_tiles = (int)((per + t.n - 1) / t.n);  // parts rounded to 32 may be fewer
     t.box = t.n / 2;
-    total = cols * t.row_tiles;
+    most = total = cols * t.row_tiles;
   }
+  if (most > (1 << 30)) return KANSO_OK;
+  t.most = (int)most;
   if (total * 4 < pairs * 3) return KANSO_OK;
   CUtensorMap wm, um, xm;
   int32_t st = weight_map(ctx, w, &wm, up ? 64 : 128);
