@@ -116,7 +116,9 @@ def test_runs_across_tiles(ctx, kb, oracle, torch_cuda, fmt, M, N, K):
 # Matrices whose K stays whole: 93 tiles of 112 rows, 148 of 128, and a K of fewer than four units
 @pytest.mark.parametrize("M,N,K", [(24, 10400, 2048), (48, 10400, 2048), (64, 10400, 2048),
                                    (96, 10400, 2048), (33, 18944, 2304), (128, 18944, 2304),
-                                   (16, 1000, 512), (128, 300, 768), (9, 131, 256)])
+                                   (16, 1000, 512), (128, 300, 768), (9, 131, 256),
+                                   (104, 10400, 2048), (128, 10400, 2048), (90, 18944, 2304),
+                                   (112, 18944, 2304)])
 def test_q8_activations_bit_exact(ctx, kb, oracle, torch_cuda, M, N, K):
     blocks = matrix("q8_0", N, K)
     x = data(M, 1, K)[1]
@@ -125,6 +127,18 @@ def test_q8_activations_bit_exact(ctx, kb, oracle, torch_cuda, M, N, K):
     ref = oracle.gemm_q8_0(np.ascontiguousarray(blocks[pick]).reshape(-1), x, M, pick.size, K,
                            oracle.ACT_Q8)
     assert (got[:, pick] == ref).all()
+
+
+@pytest.mark.parametrize("byte", [0x80, 0x7F, 0x00])
+def test_q8_activations_largest_block_sums(ctx, kb, oracle, torch_cuda, byte):
+    """32 products of -128 or 127 with +-127 are the largest sums a block can have."""
+    M, N, K = 12, 136, 512
+    blocks = matrix("q8_0", N, K)
+    blocks.reshape(N, -1, 34)[..., 2:] = byte
+    x = np.ones((M, K), np.float32)
+    x[1::2] = -3.0
+    got = several_calls(ctx, kb, torch_cuda, "q8_0", blocks, x, N, kb.ACT_Q8, 1)[0]
+    assert (got == oracle.gemm_q8_0(blocks.reshape(-1), x, M, N, K, oracle.ACT_Q8)).all()
 
 
 @pytest.mark.parametrize("M,N,K", [(16, 8000, 2048), (33, 2048, 1280)])
