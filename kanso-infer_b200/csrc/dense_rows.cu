@@ -10,26 +10,7 @@
 namespace kanso {
 
 constexpr int DR_THREADS = 256;
-
-template <typename E>
-__global__ void embed_scaled_kernel(const E* __restrict__ embed, int64_t ld,
-                                    const uint32_t* __restrict__ tokens, int64_t vocab,
-                                    float scale, float* __restrict__ x, int width,
-                                    E* __restrict__ xe, int* status) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int64_t t = blockIdx.x;
-  uint32_t id = tokens[t];
-  if (id >= vocab) {
-    if (threadIdx.x == 0) atomicOr(status, DEV_BAD_INDEX);
-    id = 0;
-  }
-  for (int i = threadIdx.x; i < ld; i += blockDim.x) {
-    const float v = i < width ? from_elem(embed[(int64_t)id * ld + i]) * scale : 0.f;
-    if (i < width) x[t * width + i] = v;
-    if (xe) xe[t * ld + i] = to_elem<E>(v);
-  }
-}
+constexpr int DR_KEEP = 2;  // float4 of a row that a thread keeps
 
 __device__ __forceinline__ void add4(float4& a, const float4& b) {
   a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w;
@@ -47,19 +28,120 @@ __device__ __forceinline__ void store4(float* p, float a, float b, float c, floa
 }
 
 template <typename E>
+__global__ void embed_scaled_kernel(const E* __restrict__ embed, int64_t ld,
+                                    const uint32_t* __restrict__ tokens, int64_t vocab,
+                                    float scale, float* __restrict__ x, int width,
+                                    E* __restrict__ xe, int* status) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t t = blockIdx.x;
+  uint32_t id = tokens[t];
+  if (id >= vocab) {
+    if (threadIdx.x == 0) atomicOr(status, DEV_BAD_INDEX);
+    id = 0;
+  }
+  if constexpr (sizeof(E) == 2) {
+    if (width % 8 == 0) {  // eight columns at a time; a row is as long as its leading dimension
+      for (int i = threadIdx.x * 8; i < width; i += (int)blockDim.x * 8) {
+        const uint4 w = *reinterpret_cast<const uint4*>(embed + (int64_t)id * ld + i);
+        float v[8];
+        unpack_bf16x2(w.x, v[0], v[1]);
+        unpack_bf16x2(w.y, v[2], v[3]);
+        unpack_bf16x2(w.z, v[4], v[5]);
+        unpack_bf16x2(w.w, v[6], v[7]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= scale;
+        store4(x + t * width + i, v[0], v[1], v[2], v[3]);
+        store4(x + t * width + i + 4, v[4], v[5], v[6], v[7]);
+        if (xe) {
+          store4(xe + t * ld + i, v[0], v[1], v[2], v[3]);
+          store4(xe + t * ld + i + 4, v[4], v[5], v[6], v[7]);
+        }
+      }
+      return;
+    }
+  }
+  for (int i = threadIdx.x; i < ld; i += blockDim.x) {
+    const float v = i < width ? from_elem(embed[(int64_t)id * ld + i]) * scale : 0.f;
+    if (i < width) x[t * width + i] = v;
+    if (xe) xe[t * ld + i] = to_elem<E>(v);
+  }
+}
+
+template <typename E>
 __global__ void __launch_bounds__(DR_THREADS)
     residual_norm_kernel(float* __restrict__ x, int width, const ResidualSource s,
                          const float* __restrict__ w, float eps, float mult, Residual form,
                          E* __restrict__ xe, int64_t xe_ld) {
   extern __shared__ __align__(16) float v[];  // [width]
   __shared__ float red[32];
-  pdl_launch_dependents();
-  pdl_wait();
   const int64_t t = blockIdx.x;
   float* xr = x + t * width;
   const bool after = form == Residual::kAddNorm;  // the norm is of the sum
   const bool four = width % 4 == 0 && s.part_stride % 4 == 0;
   float ss = 0.f;
+  if (four && width <= DR_KEEP * DR_THREADS * 4) {
+    // A thread keeps its columns between the passes and asks for everything at once: what a row takes is
+    // the latency of its loads, and the norm's weights are there before the wait. 2048 rows of 2048 17 us and
+    // 16 so (at their bytes where four experts are added), eight rows 4.8 and 3.5.
+    float4 y[DR_KEEP], r[DR_KEEP], k[DR_KEEP];
+#pragma unroll
+    for (int c = 0; c < DR_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      y[c] = r[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < width) k[c] = *reinterpret_cast<const float4*>(w + i);
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+#pragma unroll
+    for (int c = 0; c < DR_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      if (i < width) r[c] = *reinterpret_cast<const float4*>(xr + i);
+    }
+    const int terms = s.slot ? s.top : s.parts;
+#pragma unroll 4
+    for (int j = 0; j < terms; ++j) {
+      const float by = s.slot ? s.weight[t * s.top + j] : 1.f;
+      const float* src = s.slot ? s.y + (int64_t)s.slot[t * s.top + j] * width
+                                : s.y + j * s.part_stride + t * width;
+#pragma unroll
+      for (int c = 0; c < DR_KEEP; ++c) {
+        const int i = (threadIdx.x + c * DR_THREADS) * 4;
+        if (i >= width) continue;
+        const float4 u = *reinterpret_cast<const float4*>(src + i);
+        y[c].x = fmaf(by, u.x, y[c].x), y[c].y = fmaf(by, u.y, y[c].y);
+        y[c].z = fmaf(by, u.z, y[c].z), y[c].w = fmaf(by, u.w, y[c].w);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < DR_KEEP; ++c) {
+      if (after) {
+        y[c].x = fmaf(mult, r[c].x, y[c].x), y[c].y = fmaf(mult, r[c].y, y[c].y);
+        y[c].z = fmaf(mult, r[c].z, y[c].z), y[c].w = fmaf(mult, r[c].w, y[c].w);
+      }
+      ss += sum_sq4(y[c]);
+    }
+    ss = block_sum(ss, red);
+    const float inv = 1.0f / sqrtf(ss / (float)width + eps);
+#pragma unroll
+    for (int c = 0; c < DR_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      if (i >= width) continue;
+      float4 n = make_float4(y[c].x * inv * k[c].x, y[c].y * inv * k[c].y, y[c].z * inv * k[c].z,
+                             y[c].w * inv * k[c].w);
+      if (!after) {
+        n.x = r[c].x + mult * n.x, n.y = r[c].y + mult * n.y;
+        n.z = r[c].z + mult * n.z, n.w = r[c].w + mult * n.w;
+      }
+      *reinterpret_cast<float4*>(xr + i) = n;
+      if (xe) store4(xe + t * xe_ld + i, n.x, n.y, n.z, n.w);
+    }
+    if (xe)
+      for (int i = width + threadIdx.x; i < xe_ld; i += DR_THREADS) xe[t * xe_ld + i] = to_elem<E>(0.f);
+    return;
+  }
+  pdl_launch_dependents();
+  pdl_wait();
   if (four) {
 #pragma unroll 2
     for (int i = threadIdx.x * 4; i < width; i += DR_THREADS * 4) {
@@ -147,18 +229,56 @@ __global__ void __launch_bounds__(DR_THREADS)
     o[i] = to_elem<E>(i < width ? xr[i] * inv * w[i] : 0.f);
 }
 
+// Two sums over the CTA at once.
+__device__ __forceinline__ void block_sum2(float& a, float& b, float* ra, float* rb) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+    b += __shfl_xor_sync(0xFFFFFFFFu, b, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    ra[threadIdx.x >> 5] = a;
+    rb[threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  a = b = 0.f;
+#pragma unroll
+  for (int i = 0; i < DR_THREADS / 32; ++i) {
+    a += ra[i];
+    b += rb[i];
+  }
+}
+
+constexpr int QK_KEEP = 3;
 template <typename E>
 __global__ void __launch_bounds__(DR_THREADS)
     qk_norm_store_kernel(const QkvSource s, const KvDenseLayer kv, int H, const RowMap map,
                          E* __restrict__ q_out, int* status) {
-  __shared__ float red[32];
-  pdl_launch_dependents();
-  pdl_wait();
+  __shared__ float red[32], red2[32];
   const int64_t t = blockIdx.x;
   const int D = kv.k_dim, DV = kv.v_dim, G = kv.kv_heads;
   const int nq = H * D, nk = G * D, nv = G * DV;
   const int64_t width = nq + nk + nv;
   const float* src = s.qkv + t * width;
+  const bool vec = D % 8 == 0 && DV % 8 == 0 && s.part_stride % 4 == 0;
+  // a thread keeps its columns; their norms' weights are there before the wait
+  const bool keep = vec && width <= QK_KEEP * DR_THREADS * 4;
+  float4 val[QK_KEEP], nw[QK_KEEP];
+  if (keep)
+#pragma unroll
+    for (int c = 0; c < QK_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      if (i < nq + nk)
+        nw[c] = *reinterpret_cast<const float4*>(i < nq ? s.q_norm + i : s.k_norm + i - nq);
+    }
+  pdl_launch_dependents();
+  pdl_wait();
+  if (keep)
+#pragma unroll
+    for (int c = 0; c < QK_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      if (i < width) val[c] = *reinterpret_cast<const float4*>(src + i);
+    }
   auto value = [&](int i) {
     float v = src[i];
     for (int p = 1; p < s.parts; ++p) v += src[p * s.part_stride + i];
@@ -173,7 +293,43 @@ __global__ void __launch_bounds__(DR_THREADS)
   if (!ok && threadIdx.x == 0) atomicOr(status, DEV_BAD_INDEX);
   E* pool = reinterpret_cast<E*>(kv.base);
 
-  if (D % 8 == 0 && DV % 8 == 0 && s.part_stride % 4 == 0) {
+  if (keep) {
+    float sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int c = 0; c < QK_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      if (i >= width) continue;
+      for (int p = 1; p < s.parts; ++p)
+        add4(val[c], *reinterpret_cast<const float4*>(src + p * s.part_stride + i));
+      if (i < nq)
+        sq += sum_sq4(val[c]);
+      else if (i < nq + nk)
+        sk += sum_sq4(val[c]);
+    }
+    block_sum2(sq, sk, red, red2);
+    const float iq = 1.0f / sqrtf(sq / (float)nq + s.eps), ik = 1.0f / sqrtf(sk / (float)nk + s.eps);
+#pragma unroll
+    for (int c = 0; c < QK_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      if (i >= width) continue;
+      float4 v = val[c];
+      if (i < nq + nk) {
+        const float f = i < nq ? iq : ik;
+        v.x *= f * nw[c].x, v.y *= f * nw[c].y, v.z *= f * nw[c].z, v.w *= f * nw[c].w;
+      }
+      E* dst = q_out + t * nq + i;
+      if (i >= nq + nk) {
+        const int j = i - nq - nk, g = j / DV;
+        dst = pool + kv.v_elem(ok ? block : 0u, g, off) + (j - g * DV);
+      } else if (i >= nq) {
+        const int j = i - nq, g = j / D;
+        dst = pool + kv.k_elem(ok ? block : 0u, g, off) + (j - g * D);
+      }
+      if (ok || i < nq) store4(dst, v.x, v.y, v.z, v.w);
+    }
+    return;
+  }
+  if (vec) {
     // rows without pads, four columns at a time; the sums of the parts stay in shared memory
     extern __shared__ __align__(16) float row[];  // [width]
     float sq = 0.f, sk = 0.f;
@@ -259,40 +415,71 @@ __global__ void expert_sum_kernel(const float* __restrict__ ye, const uint32_t* 
 // Router and choice, one CTA per RW rows: its warps share out the experts, two at a time
 // (logits = router . x + bias in f32), then one warp per row makes the choice (warp_route).
 template <int RW>
-__global__ void __launch_bounds__(DR_THREADS)
+__global__ void __launch_bounds__(DR_THREADS, RW == 1 ? 1 : 4)
     route_kernel(const float* __restrict__ x, int width, const float* __restrict__ router, int ld,
                  const float* __restrict__ bias, int experts, int top, RouteWeights form, uint32_t* __restrict__ sel, float* __restrict__ weight,
                  uint32_t* __restrict__ counts, uint32_t* __restrict__ slot, int64_t T) {
   extern __shared__ __align__(16) float sm[];
-  pdl_launch_dependents();
-  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t t0 = (int64_t)blockIdx.x * RW;
   float* xw = sm;             // [RW][ld]
   float* l = xw + RW * ld;    // [RW][experts]
+  // Columns of two experts' weights, AHEAD x 128 at a time; the first of them before the wait. One row per
+  // CTA is all latency and takes what 2048 columns have in one go.
+  constexpr int AHEAD = RW == 1 ? 16 : 4;
+  float4 a[AHEAD], b[AHEAD];
+  auto fetch = [&](int e0, int c0) {
+    const float* w0 = router + (int64_t)e0 * ld + c0 + lane * 4;
+    const float* w1 = router + (int64_t)min(e0 + 1, experts - 1) * ld + c0 + lane * 4;
 #pragma unroll
-  for (int r = 0; r < RW; ++r)
-    for (int i = threadIdx.x; i < ld; i += DR_THREADS)
-      xw[r * ld + i] = i < width && t0 + r < T ? x[(t0 + r) * width + i] : 0.f;
+    for (int k = 0; k < AHEAD; ++k) {
+      a[k] = b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c0 + k * 128 + lane * 4 < ld) {
+        a[k] = __ldg(reinterpret_cast<const float4*>(w0 + k * 128));
+        b[k] = __ldg(reinterpret_cast<const float4*>(w1 + k * 128));
+      }
+    }
+  };
+  if (warp * 2 < experts) fetch(warp * 2, 0);
+  pdl_launch_dependents();
+  pdl_wait();
+  if (width % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+#pragma unroll 2
+    for (int i = threadIdx.x * 4; i < ld; i += DR_THREADS * 4) {
+      float4 v[RW];
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+        v[r] = i < width && t0 + r < T ? *reinterpret_cast<const float4*>(x + (t0 + r) * width + i)
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < RW; ++r) *reinterpret_cast<float4*>(xw + r * ld + i) = v[r];
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+      for (int i = threadIdx.x; i < ld; i += DR_THREADS)
+        xw[r * ld + i] = i < width && t0 + r < T ? x[(t0 + r) * width + i] : 0.f;
+  }
   __syncthreads();
   for (int e0 = warp * 2; e0 < experts; e0 += DR_THREADS / 32 * 2) {
-    const float* w0 = router + (int64_t)e0 * ld;
-    const float* w1 = router + (int64_t)min(e0 + 1, experts - 1) * ld;
     float acc[RW * 2];
 #pragma unroll
     for (int i = 0; i < RW * 2; ++i) acc[i] = 0.f;
-#pragma unroll 4
-    for (int c = lane * 4; c < ld; c += 128) {
-      const float4 a = *reinterpret_cast<const float4*>(w0 + c);
-      const float4 b = *reinterpret_cast<const float4*>(w1 + c);
+    for (int c0 = 0; c0 < ld; c0 += AHEAD * 128) {
+      if (c0 || e0 != warp * 2) fetch(e0, c0);
 #pragma unroll
-      for (int r = 0; r < RW; ++r) {
-        const float4 v = *reinterpret_cast<const float4*>(xw + r * ld + c);
-        float s = acc[r * 2], u = acc[r * 2 + 1];
-        s = fmaf(a.x, v.x, s), u = fmaf(b.x, v.x, u);
-        s = fmaf(a.y, v.y, s), u = fmaf(b.y, v.y, u);
-        s = fmaf(a.z, v.z, s), u = fmaf(b.z, v.z, u);
-        acc[r * 2] = fmaf(a.w, v.w, s), acc[r * 2 + 1] = fmaf(b.w, v.w, u);
+      for (int k = 0; k < AHEAD; ++k) {
+        const int c = c0 + k * 128 + lane * 4;
+        if (c >= ld) continue;
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const float4 v = *reinterpret_cast<const float4*>(xw + r * ld + c);
+          float s = acc[r * 2], u = acc[r * 2 + 1];
+          s = fmaf(a[k].x, v.x, s), u = fmaf(b[k].x, v.x, u);
+          s = fmaf(a[k].y, v.y, s), u = fmaf(b[k].y, v.y, u);
+          s = fmaf(a[k].z, v.z, s), u = fmaf(b[k].z, v.z, u);
+          acc[r * 2] = fmaf(a[k].w, v.w, s), acc[r * 2 + 1] = fmaf(b[k].w, v.w, u);
+        }
       }
     }
 #pragma unroll
