@@ -1,6 +1,7 @@
 // Unquantised (bfloat16 or f32) layers: what the row-streaming kernels, the tile kernels, the
 // expert routing, the attentions and the recurrence share, and their launchers.
 #pragma once
+#include <algorithm>
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -206,6 +207,15 @@ struct GemmOut {
   int64_t group_step = 0;
   const uint32_t* rows = nullptr;  // with group_step: row r of a group goes to row rows[r]
 };
+// How many parts a model asks for at most in a step of T rows, and the rows that the results of all
+// parts come to: workspaces are made for the largest step, and smaller ones fit the same parts into them.
+// (Parts once depended on the rows the workspace was made for: behind a long prompt eight decoding rows had
+// one, and 3072 x 2048 on 24 SMs took 11 us, 6 in four parts; eight parts cost their readers what they save.)
+inline int split_parts(int64_t T) { return T <= 512 ? 4 : 1; }
+inline int64_t split_rows(int64_t T) {
+  return std::max<int64_t>(T, 4 * std::min<int64_t>(T, 512));
+}
+
 // y[T][rows] = x[T][ld] W^T, f32 unless `o` says otherwise. With *splits > 1 on return the result
 // is the sum of that many arrays [T][y_ld], `part_stride` elements apart (only when max_splits
 // allows it).

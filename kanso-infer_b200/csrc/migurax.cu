@@ -142,7 +142,6 @@ struct MiguraxModel final : DenseModel {
   DenseMat embed, head;
   float* final_norm = nullptr;
   // workspace of `ws_rows` rows
-  int ws_parts = 1;
   float *x = nullptr, *x2 = nullptr, *y = nullptr, *q = nullptr, *q_lat = nullptr,
         *o_lat32 = nullptr, *mix32 = nullptr, *act32 = nullptr, *oy = nullptr, *ye = nullptr,
         *rl = nullptr, *wgt = nullptr;
@@ -315,7 +314,7 @@ int32_t MiguraxModel::load(const SafeTensors& st) {
 
 int32_t MiguraxModel::ensure_ws(int64_t T) {
   if (T <= ws_rows) return KANSO_OK;
-  ws_parts = T <= 512 ? 4 : 1;
+  const int64_t split = split_rows(T);
   int64_t ny = 0, nq = 0, n_cq = 0, n_qh = 0, n_qr = 0, n_lat = 0, n_o = 0, nact = 0, ne = 0, nt = 1;
   size_t chunk = 0;
   for (const MigLayerSpec& s : cfg.layers) {
@@ -340,13 +339,13 @@ int32_t MiguraxModel::ensure_ws(int64_t T) {
   counts_bytes = cfg.layers.size() * (size_t)ne * 4;
   return make_ws(T, {{(void**)&x, (size_t)(T * W) * 4},
                      {(void**)&x2, (size_t)(T * W) * 4},
-                     {(void**)&y, (size_t)(ws_parts * T * ny) * 4},
-                     {(void**)&q, (size_t)(ws_parts * T * nq) * 4},
+                     {(void**)&y, (size_t)(split * ny) * 4},
+                     {(void**)&q, (size_t)(split * nq) * 4},
                      {(void**)&q_lat, (size_t)(T * n_lat) * 4},
                      {(void**)&o_lat32, (size_t)(few * n_lat) * 4},
                      {(void**)&mix32, (size_t)(T * n_o) * 4},
                      {(void**)&act32, (size_t)(few * nact) * 4},
-                     {(void**)&oy, (size_t)(ws_parts * T * W) * 4},
+                     {(void**)&oy, (size_t)(split * W) * 4},
                      {(void**)&ye, (size_t)(T * nt * W) * 4},
                      {(void**)&rl, (size_t)(few * ne) * 4},
                      {(void**)&wgt, (size_t)(T * nt) * 4},
@@ -629,7 +628,7 @@ int32_t MiguraxModel::latent_tiles(kanso_cuda_kv* kv, size_t l, const DenseStep&
   const MigLayer& ly = layers[l];
   const MigLayerSpec& sp = cfg.layers[l];
   const int64_t T = s.T;
-  const int max_splits = T <= 512 ? ws_parts : 1;
+  const int max_splits = split_parts(T);
   GemmRows rows;
   rows.T = T;
   int32_t st;
@@ -665,7 +664,7 @@ int32_t MiguraxModel::memory_tiles(kanso_cuda_kv* kv, size_t l, const DenseStep&
   rows.T = s.T;
   int32_t st;
   int parts = 1;
-  if ((st = launch_gemm(ctx, compute, ly.in, xe, y, ly.in.rows, rows, s.T <= 512 ? ws_parts : 1,
+  if ((st = launch_gemm(ctx, compute, ly.in, xe, y, ly.in.rows, rows, split_parts(s.T),
                         &parts, s.T * ly.in.rows)))
     return st;
   const MlstmArgs a = memory_of(kv, l, s, parts);
@@ -686,7 +685,7 @@ int32_t MiguraxModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
   const int64_t T = s.T, W = cfg.width, WL = round_up8(W);
   int32_t st;
   int splits = 1;
-  const int max_splits = T <= 512 ? ws_parts : 1;
+  const int max_splits = split_parts(T);
   GemmRows rows;
   rows.T = T;
   if ((st = launch_embed_scaled(ctx, compute, embed.w, embed.ld, s.tokens, cfg.vocab, 1.f, x, W, xe,

@@ -102,7 +102,6 @@ struct RevitarModel final : DenseModel {
   DenseMat embed, head;
   float* final_norm = nullptr;
   // workspace of `ws_rows` rows
-  int ws_parts = 1;
   float *x = nullptr, *x2 = nullptr, *qkv = nullptr, *oy = nullptr, *ao32 = nullptr,
         *rl = nullptr, *wgt = nullptr, *act32 = nullptr, *ye = nullptr;
   void *xe = nullptr, *q = nullptr, *ao = nullptr, *xs = nullptr, *act = nullptr;
@@ -184,7 +183,7 @@ int32_t RevitarModel::load(const SafeTensors& st) {
 
 int32_t RevitarModel::ensure_ws(int64_t T) {
   if (T <= ws_rows) return KANSO_OK;
-  ws_parts = T <= 512 ? 4 : 1;
+  const int64_t split = split_rows(T);
   int64_t n_qkv = 0, n_q = 0, n_o = 0, ne = 0, nt = 0, nact = 0, nact32 = 0;
   for (const RevLayerSpec& s : cfg.layers) {
     n_qkv = std::max(n_qkv, (int64_t)s.heads * s.dim + (int64_t)s.kv_heads * (s.dim + s.vdim));
@@ -201,8 +200,8 @@ int32_t RevitarModel::ensure_ws(int64_t T) {
   return make_ws(T,
               {{(void**)&x, (size_t)(T * W) * 4},
                {(void**)&x2, (size_t)(T * W) * 4},
-               {(void**)&qkv, (size_t)(ws_parts * T * n_qkv) * 4},
-               {(void**)&oy, (size_t)(ws_parts * T * W) * 4},
+               {(void**)&qkv, (size_t)(split * n_qkv) * 4},
+               {(void**)&oy, (size_t)(split * W) * 4},
                {(void**)&ao32, (size_t)(std::min<int64_t>(T, GEMV_MAX_T) * n_o) * 4},
                {(void**)&act32, (size_t)(std::min<int64_t>(T, GEMV_MAX_T) * nact32) * 4},
                {(void**)&rl, (size_t)(std::min<int64_t>(T, GEMV_MAX_T) * ne) * 4},
@@ -327,7 +326,7 @@ int32_t RevitarModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
   const int64_t T = s.T, W = cfg.width, WL = round_up8(W);
   int32_t st;
   int splits = 1;
-  const int max_splits = T <= 512 ? ws_parts : 1;
+  const int max_splits = split_parts(T);
   GemmRows rows;
   rows.T = T;
   if ((st = launch_embed_scaled(ctx, compute, embed.w, embed.ld, s.tokens, cfg.vocab,
