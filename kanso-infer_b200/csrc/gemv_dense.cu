@@ -171,10 +171,212 @@ __device__ __forceinline__ void gate_source(const GemvSource& s, const float* x,
   }
 }
 
+__device__ __forceinline__ bool aligned16_dev(const void* p) {
+  return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
+}
+__device__ __forceinline__ float4 f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+// Sums of TT values over the CTA; every thread gets them.
+template <int TT>
+__device__ __forceinline__ void block_sums(float (&v)[TT], float* red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < TT; ++t) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v[t] += __shfl_xor_sync(0xFFFFFFFFu, v[t], o);
+    if (lane == 0) red[warp * TT + t] = v[t];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < TT; ++t) {
+    v[t] = 0.f;
+#pragma unroll
+    for (int w = 0; w < GV_WARPS; ++w) v[t] += red[w * TT + t];
+  }
+  __syncthreads();
+}
+
+// gate_source for all rows at once, heads of whole 128 columns: a warp's lanes read 128 neighbours.
+template <int TT>
+__device__ __forceinline__ bool gate_source_wide(const GemvSource& s, int cols, int ld, int t0, int nt,
+                                                 float* xs, float* red) {
+  constexpr int KEEP = 2, CHUNKS = KEEP * GV_WARPS;  // 128 columns each
+  const int hd = cols / s.heads, per = hd / 128, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (hd % 128 || cols > CHUNKS * 128 || s.gate_ld % 4 || s.part_stride % 4 || !aligned16_dev(s.x) ||
+      !aligned16_dev(s.gate) || !aligned16_dev(s.norm_w))
+    return false;
+  float4 v[TT][KEEP], g[TT][KEEP], k[KEEP];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < KEEP; ++c) {
+    const int i = (threadIdx.x + c * GV_THREADS) * 4;
+    k[c] = i < cols ? f4(s.norm_w + i) : zero;
+#pragma unroll
+    for (int t = 0; t < TT; ++t) {
+      const bool in = t < nt && i < cols;
+      const int64_t r = s.row_index && t < nt ? s.row_index[t0 + t] : t0 + t;
+      v[t][c] = in ? f4(s.x + r * cols + i) : zero;
+      g[t][c] = in ? f4(s.gate + r * s.gate_ld + i) : zero;
+    }
+  }
+  for (int p = 1; p < s.parts; ++p)
+#pragma unroll
+    for (int c = 0; c < KEEP; ++c)
+#pragma unroll
+      for (int t = 0; t < TT; ++t) {
+        const int i = (threadIdx.x + c * GV_THREADS) * 4;
+        if (t >= nt || i >= cols) continue;
+        const int64_t r = s.row_index ? s.row_index[t0 + t] : t0 + t;
+        const float4 u = f4(s.gate + p * s.part_stride + r * s.gate_ld + i);
+        g[t][c].x += u.x, g[t][c].y += u.y, g[t][c].z += u.z, g[t][c].w += u.w;
+      }
+#pragma unroll
+  for (int t = 0; t < TT; ++t)
+#pragma unroll
+    for (int c = 0; c < KEEP; ++c) {
+      const float4& a = v[t][c];
+      float ss = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+#pragma unroll
+      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+      if (lane == 0) red[t * CHUNKS + c * GV_WARPS + warp] = ss;
+    }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < TT; ++t)
+#pragma unroll
+    for (int c = 0; c < KEEP; ++c) {
+      const int i = (threadIdx.x + c * GV_THREADS) * 4, h = (c * GV_WARPS + warp) / per;
+      if (i >= cols) continue;
+      float ss = 0.f;
+      for (int q = 0; q < per; ++q) ss += red[t * CHUNKS + h * per + q];
+      const float inv = 1.0f / sqrtf(ss / (float)hd + s.eps);
+      const float4 &a = v[t][c], &b = g[t][c], &n = k[c];
+      *reinterpret_cast<float4*>(xs + t * ld + ((i >> 2) & 1) * (ld >> 1) + (i >> 3) * 4) =
+          make_float4(a.x * n.x / (1.0f + expf(-b.x)) * inv, a.y * n.y / (1.0f + expf(-b.y)) * inv,
+                      a.z * n.z / (1.0f + expf(-b.z)) * inv, a.w * n.w / (1.0f + expf(-b.w)) * inv);
+    }
+  __syncthreads();
+  return true;
+}
+
+// The same as norm_source for rows of whole float4: all rows at once, and what a thread works on stays in
+// registers. Every CTA of a product forms its input, so that its latency is the product's: with one row, one
+// float and one pass after another 4096 x 2048 behind a residual step took 19.3 us at two rows, 12.2 so, and 9.4
+// once every CTA stays for the whole product (gv_grid).
+constexpr int GV_KEEP = 2;  // float4 of a row that a thread keeps
+template <int TT, int KIND>
+__device__ __forceinline__ bool norm_source_wide(const GemvSource& s, int cols, int ld, int t0, int nt,
+                                                 bool writer, float* xs, float* red) {
+  const bool step = KIND != GV_GROUPS_IN && s.y;
+  if (KIND == GV_GATED_IN || cols % 8 || !aligned16_dev(s.x) || (step && cols > GV_KEEP * GV_THREADS * 4) ||
+      (KIND == GV_GROUPS_IN && (s.x_ld % 4 || s.x_group % 4)) ||
+      (step && (!aligned16_dev(s.y) || s.part_stride % 4 || !aligned16_dev(s.norm_w))) ||
+      (s.final_w && (!step || !aligned16_dev(s.final_w))) || (s.x_out && !aligned16_dev(s.x_out)))
+    return false;
+  const float* x[TT];
+  int64_t row[TT];
+#pragma unroll
+  for (int t = 0; t < TT; ++t) {
+    const int64_t r = s.row_index && t < nt ? s.row_index[t0 + t] : t0 + t;
+    row[t] = r * cols;
+    x[t] = KIND == GV_GROUPS_IN ? s.x + r * s.x_ld + blockIdx.z * s.x_group : s.x + r * cols;
+  }
+  auto put = [&](int t, int i, const float4& v) {
+    *reinterpret_cast<float4*>(xs + t * ld + ((i >> 2) & 1) * (ld >> 1) + (i >> 3) * 4) = v;
+  };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!step) {
+#pragma unroll 4
+    for (int i = threadIdx.x * 4; i < cols; i += GV_THREADS * 4)
+#pragma unroll
+      for (int t = 0; t < TT; ++t) {
+        const float4 v = t < nt ? f4(x[t] + i) : zero;
+        if (writer && s.x_out && t < nt) *reinterpret_cast<float4*>(s.x_out + row[t] + i) = v;
+        put(t, i, v);
+      }
+    return true;
+  }
+  const bool after = KIND == GV_ROWS_IN && s.form == Residual::kAddNorm;
+  float4 v[TT][GV_KEEP], old[TT][GV_KEEP], k[GV_KEEP];
+  float ss[TT];
+#pragma unroll
+  for (int c = 0; c < GV_KEEP; ++c) {
+    const int i = (threadIdx.x + c * GV_THREADS) * 4;
+    k[c] = i < cols ? f4(s.norm_w + i) : zero;
+#pragma unroll
+    for (int t = 0; t < TT; ++t) {
+      const bool in = t < nt && i < cols;
+      v[t][c] = in ? f4(s.y + row[t] + i) : zero;
+      old[t][c] = in ? f4(x[t] + i) : zero;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < TT; ++t) {
+    ss[t] = 0.f;
+#pragma unroll
+    for (int c = 0; c < GV_KEEP; ++c) {
+      const int i = (threadIdx.x + c * GV_THREADS) * 4;
+      float4& a = v[t][c];
+      if (t < nt && i < cols)
+        for (int p = 1; p < s.parts; ++p) {
+          const float4 u = f4(s.y + p * s.part_stride + row[t] + i);
+          a.x += u.x, a.y += u.y, a.z += u.z, a.w += u.w;
+        }
+      const float4& o = old[t][c];
+      if (after) {
+        a.x = fmaf(s.mult, o.x, a.x), a.y = fmaf(s.mult, o.y, a.y);
+        a.z = fmaf(s.mult, o.z, a.z), a.w = fmaf(s.mult, o.w, a.w);
+      }
+      ss[t] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+    }
+  }
+  block_sums(ss, red);
+  float s2[TT];
+#pragma unroll
+  for (int t = 0; t < TT; ++t) {
+    const float inv = 1.0f / sqrtf(ss[t] / (float)cols + s.eps);
+    s2[t] = 0.f;
+#pragma unroll
+    for (int c = 0; c < GV_KEEP; ++c) {
+      const int i = (threadIdx.x + c * GV_THREADS) * 4;
+      float4& a = v[t][c];
+      const float4& o = old[t][c];
+      a = make_float4(a.x * inv * k[c].x, a.y * inv * k[c].y, a.z * inv * k[c].z, a.w * inv * k[c].w);
+      if (!after) {
+        a.x = o.x + s.mult * a.x, a.y = o.y + s.mult * a.y;
+        a.z = o.z + s.mult * a.z, a.w = o.w + s.mult * a.w;
+      }
+      if (i < cols) {
+        if (writer && s.x_out && t < nt) *reinterpret_cast<float4*>(s.x_out + row[t] + i) = a;
+        if (!s.final_w) put(t, i, t < nt ? a : zero);
+      }
+      s2[t] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+    }
+  }
+  if (!s.final_w) return true;
+  block_sums(s2, red);
+#pragma unroll
+  for (int c = 0; c < GV_KEEP; ++c) {
+    const int i = (threadIdx.x + c * GV_THREADS) * 4;
+    if (i >= cols) continue;
+    const float4 f = f4(s.final_w + i);
+#pragma unroll
+    for (int t = 0; t < TT; ++t) {
+      const float inv = 1.0f / sqrtf(s2[t] / (float)cols + s.eps);
+      const float4& a = v[t][c];
+      put(t, i, t < nt ? make_float4(a.x * inv * f.x, a.y * inv * f.y, a.z * inv * f.z, a.w * inv * f.w)
+                       : zero);
+    }
+  }
+  return true;
+}
+
 // The input rows of this CTA, into shared memory (and the residual step's to x_out by one CTA).
 template <int TT, int KIND>
 __device__ __forceinline__ void norm_source(const GemvSource& s, int cols, int ld, int t0, int nt,
                                             bool writer, float* xs, float* red) {
+  if (KIND == GV_GATED_IN ? gate_source_wide<TT>(s, cols, ld, t0, nt, xs, red)
+                          : norm_source_wide<TT, KIND>(s, cols, ld, t0, nt, writer, xs, red))
+    return;
   for (int t = 0; t < nt; ++t) {
     const int64_t r = s.row_index ? s.row_index[t0 + t] : t0 + t;
     const float* x = s.x + r * cols;
@@ -298,7 +500,7 @@ struct GateUpArgs {
 // Two gate rows and the two up rows beside them per warp step, without a gate four up rows;
 // blockIdx.y = row * top + place.
 template <typename E, bool GATED>
-__global__ void __launch_bounds__(GV_THREADS) gemv_gate_up_kernel(const GateUpArgs a) {
+__global__ void __launch_bounds__(GV_THREADS, sizeof(E) == 2 ? 4 : 2) gemv_gate_up_kernel(const GateUpArgs a) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[GV_WARPS * GV_ROWS];
   float* xs = sm;                          // [ld]
@@ -309,12 +511,20 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_gate_up_kernel(const GateUpAr
   const int t = blockIdx.y / a.top, place = blockIdx.y % a.top;
   pdl_launch_dependents();
   pdl_wait();
-  for (int e = threadIdx.x; e < a.experts; e += GV_THREADS)
-    lg[e] = a.logits[(int64_t)t * a.experts + e];
-  for (int i = threadIdx.x; i < a.ld; i += GV_THREADS)
-    xs[xs_index(i, a.ld)] = i < a.cols ? a.x[(int64_t)t * a.cols + i] : 0.f;
-  __syncthreads();
-  if (warp == 0) warp_route(lg, a.experts, a.top, a.form, lane, sel, wt);
+  // one warp chooses while the others fetch the row
+  if (warp == 0) {
+    for (int e = lane; e < a.experts; e += 32) lg[e] = a.logits[(int64_t)t * a.experts + e];
+    __syncwarp();
+    warp_route(lg, a.experts, a.top, a.form, lane, sel, wt);
+  } else if (a.cols % 8 == 0 && aligned16_dev(a.x)) {
+#pragma unroll 4
+    for (int i = (threadIdx.x - 32) * 4; i < a.cols; i += (GV_THREADS - 32) * 4)
+      *reinterpret_cast<float4*>(xs + ((i >> 2) & 1) * (a.ld >> 1) + (i >> 3) * 4) =
+          f4(a.x + (int64_t)t * a.cols + i);
+  } else {
+    for (int i = threadIdx.x - 32; i < a.ld; i += GV_THREADS - 32)
+      xs[xs_index(i, a.ld)] = i < a.cols ? a.x[(int64_t)t * a.cols + i] : 0.f;
+  }
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) a.sel[blockIdx.y] = sel[place];
   const float weight = wt[place];
@@ -365,15 +575,24 @@ struct DownArgs {
 
 // blockIdx.y = row of the step; the columns are the chosen experts' one after the other.
 template <typename E>
-__global__ void __launch_bounds__(GV_THREADS) gemv_down_kernel(const DownArgs a) {
+__global__ void __launch_bounds__(GV_THREADS, sizeof(E) == 2 ? 4 : 2) gemv_down_kernel(const DownArgs a) {
   extern __shared__ __align__(16) float xs[];  // [top][ld], two planes each
   __shared__ float red[GV_WARPS * GV_ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.y;
   pdl_launch_dependents();
   pdl_wait();
-  for (int i = threadIdx.x; i < a.top * a.ld; i += GV_THREADS) {
-    const int j = i / a.ld, c = i - j * a.ld;
-    xs[j * a.ld + xs_index(c, a.ld)] = a.act[(int64_t)t * a.top * a.ld + i];
+  if (aligned16_dev(a.act)) {  // leading dimensions are multiples of eight
+#pragma unroll 4
+    for (int i = threadIdx.x * 4; i < a.top * a.ld; i += GV_THREADS * 4) {
+      const int j = i / a.ld, c = i - j * a.ld;
+      *reinterpret_cast<float4*>(xs + j * a.ld + ((c >> 2) & 1) * (a.ld >> 1) + (c >> 3) * 4) =
+          f4(a.act + (int64_t)t * a.top * a.ld + i);
+    }
+  } else {
+    for (int i = threadIdx.x; i < a.top * a.ld; i += GV_THREADS) {
+      const int j = i / a.ld, c = i - j * a.ld;
+      xs[j * a.ld + xs_index(c, a.ld)] = a.act[(int64_t)t * a.top * a.ld + i];
+    }
   }
   __syncthreads();
   const int gpc = GV_WARPS / a.ks, sub = warp % a.ks, per = a.ld / 8, chunks = per * a.top;
@@ -434,9 +653,11 @@ static int pick_ks(const kanso_cuda_ctx* ctx, int64_t groups, int64_t copies, in
     ks *= 2;
   return ks;
 }
-static unsigned gv_grid(const kanso_cuda_ctx* ctx, int64_t groups, int ks, int64_t copies) {
+// per_sm: CTAs that an SM holds. Where each forms the input first, more of them form it again: 512 of
+// them, 444 at a time, took 14.9 us for 2048 gated columns x 2048 rows, 444 take 8.9.
+static unsigned gv_grid(const kanso_cuda_ctx* ctx, int64_t groups, int ks, int64_t copies, int per_sm = 8) {
   const int64_t gpc = GV_WARPS / ks, need = (groups + gpc - 1) / gpc;
-  const int64_t cap = std::max<int64_t>(1, 8 * (int64_t)ctx->sm_count / copies);
+  const int64_t cap = std::max<int64_t>(1, (int64_t)per_sm * ctx->sm_count / copies);
   return (unsigned)std::min(need, cap);
 }
 
@@ -475,7 +696,8 @@ int32_t launch_gemv(kanso_cuda_ctx* ctx, int32_t compute, const DenseMat& w, con
                                pick_ks(ctx, groups, all, w.ld / 8), T, s, out, out_ld, o};
   a.store_ctas = store ? T : 0;
   if (store) a.store = *store;
-  const dim3 grid(gv_grid(ctx, groups, a.ks, all) + a.store_ctas, (unsigned)copies,
+  const int resident = compute == KANSO_COMPUTE_BF16 ? (tt == 1 ? 4 : 3) : 2;
+  const dim3 grid(gv_grid(ctx, groups, a.ks, all, resident) + a.store_ctas, (unsigned)copies,
                   (unsigned)w.groups);
   if (compute == KANSO_COMPUTE_BF16) {
     switch (tt) {

@@ -53,7 +53,12 @@ ODD = config(67, 45, [memory(3, 7, 9, dense(21)), latent(3, 9, 6, 11, 13, 11, mo
 # value columns beyond the prompt attention's, key columns beyond the chunks': other kernels step in
 LARGE = config(90, 64, [latent(3, 24, 8, 200, 40, 32, dense(64)), memory(1, 530, 24, None),
                         latent(2, 360, 16, 16, 24, 16, None)])
-MODELS = {"attention": ATTENTION, "large": LARGE, "odd": ODD, "memory": MEMORY, "mixed": MIXED, "one": ONE, "uneven": UNEVEN,
+# rows of whole 16 bytes and heads of whole 128 columns, which have forms of their own; and just wider than
+# a thread's registers hold
+BROAD = config(90, 256, [memory(2, 32, 128, dense(136)), memory(3, 16, 256, moe(4, 2, 40)),
+                         latent(4, 32, 16, 32, 64, 40, dense(128))])
+BEYOND = config(60, 2056, [memory(9, 8, 256, dense(24)), latent(2, 16, 8, 16, 24, 16, moe(3, 1, 16))])
+MODELS = {"beyond": BEYOND, "broad": BROAD, "attention": ATTENTION, "large": LARGE, "odd": ODD, "memory": MEMORY, "mixed": MIXED, "one": ONE, "uneven": UNEVEN,
           "wide": WIDE}
 
 
