@@ -639,6 +639,28 @@ __global__ void __launch_bounds__(DR_THREADS)
     for (int p = 1; p < q.parts; ++p) v += src[p * q.part_stride + i];
     return v;
   };
+  if (D % 8 == 0 && RD % 8 == 0 && q.ld % 4 == 0 && q.part_stride % 4 == 0) {  // no pads, four at a time
+    auto value4 = [&](int64_t i) {
+      float4 v = *reinterpret_cast<const float4*>(src + i);
+      for (int p = 1; p < q.parts; ++p)
+        add4(v, *reinterpret_cast<const float4*>(src + p * q.part_stride + i));
+      return v;
+    };
+#pragma unroll 2
+    for (int k = threadIdx.x * 4; k < H * D; k += DR_THREADS * 4) {
+      const int h = k / D;
+      const float4 v = value4(k + (int64_t)h * RD);
+      store4(out + t * H * D + k, v.x, v.y, v.z, v.w);
+    }
+    for (int k = threadIdx.x * 4; k < H * RD; k += DR_THREADS * 4) {
+      const int h = k / RD, d = k - h * RD;
+      const float4 v = value4(k + (int64_t)(h + 1) * D);
+      const float2 a0 = turn[d / 2], a1 = turn[d / 2 + 1];
+      store4(out_rot + t * H * RD + k, v.x * a0.y - v.y * a0.x, v.y * a0.y + v.x * a0.x,
+             v.z * a1.y - v.w * a1.x, v.w * a1.y + v.z * a1.x);
+    }
+    return;
+  }
   // two columns at a time (the leading dimensions are even)
   for (int k = threadIdx.x * 2; k < H * ld; k += DR_THREADS * 2) {
     const int h = k / ld, d = k - h * ld;
@@ -701,17 +723,36 @@ __global__ void __launch_bounds__(HN_THREADS)
                           const float* __restrict__ w, float eps, E* __restrict__ out,
                           int64_t out_ld) {
   __shared__ float red[32];
-  pdl_launch_dependents();
-  pdl_wait();
   const int h = blockIdx.x, n = heads * hd;
   const int64_t t = blockIdx.y;
   const float *x = o + t * n + h * hd, *g = gate + t * gate_ld + h * hd;
   E* dst = out + t * out_ld + h * hd;
   w += h * hd;
   float ss = 0.f;
+  const int at = threadIdx.x * 4;
+  const bool own = at < hd;  // a thread's columns of a head that has no more than four for each
+  const bool once = hd % 4 == 0 && hd <= HN_THREADS * 4;
+  float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (once && own) k4 = *reinterpret_cast<const float4*>(w + at);
+  pdl_launch_dependents();
+  pdl_wait();
   if (hd % 4 == 0 && gate_ld % 4 == 0 && part_stride % 4 == 0 &&
       ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
-      out_ld % 4 == 0) {
+      out_ld % 4 == 0 && once) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f), z = v;
+    if (own) {
+      v = *reinterpret_cast<const float4*>(x + at);
+      z = *reinterpret_cast<const float4*>(g + at);
+      for (int p = 1; p < parts; ++p) add4(z, *reinterpret_cast<const float4*>(g + p * part_stride + at));
+    }
+    ss = block_sum(sum_sq4(v), red);
+    const float inv = 1.0f / sqrtf(ss / (float)hd + eps);
+    if (own)
+      store4(dst + at, v.x * inv * k4.x / (1.0f + expf(-z.x)), v.y * inv * k4.y / (1.0f + expf(-z.y)),
+             v.z * inv * k4.z / (1.0f + expf(-z.z)), v.w * inv * k4.w / (1.0f + expf(-z.w)));
+  } else if (hd % 4 == 0 && gate_ld % 4 == 0 && part_stride % 4 == 0 &&
+             ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
+             out_ld % 4 == 0) {
     for (int i = threadIdx.x * 4; i < hd; i += HN_THREADS * 4)
       ss += sum_sq4(*reinterpret_cast<const float4*>(x + i));
     ss = block_sum(ss, red);

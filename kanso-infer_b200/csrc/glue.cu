@@ -9,11 +9,43 @@
 namespace kanso {
 
 // x / sqrt(mean(x^2) + eps) * w, one CTA per row (src/model.rs:653-659).
+constexpr int RMS_KEEP = 4;
+template <bool VEC>
 __global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                float* __restrict__ out, int hidden, float eps) {
   __shared__ float red[32];
   const float* xr = x + (int64_t)blockIdx.x * hidden;
   float ss = 0.f;
+  if (VEC) {  // hidden % 4 == 0, at most RMS_KEEP * 1024: a thread keeps its columns
+    float* o = out + (int64_t)blockIdx.x * hidden;
+    float4 v[RMS_KEEP], k[RMS_KEEP];
+    pdl_launch_dependents();
+    pdl_wait();
+#pragma unroll
+    for (int c = 0; c < RMS_KEEP; ++c) {
+      const int i = (threadIdx.x + c * 256) * 4;
+      v[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < hidden) {
+        v[c] = *reinterpret_cast<const float4*>(xr + i);
+        k[c] = *reinterpret_cast<const float4*>(w + i);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < RMS_KEEP; ++c)
+      ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
+    const float rms = sqrtf(block_sum(ss, red) / (float)hidden + eps);
+#pragma unroll
+    for (int c = 0; c < RMS_KEEP; ++c) {
+      const int i = (threadIdx.x + c * 256) * 4;
+      if (i < hidden)
+        *reinterpret_cast<float4*>(o + i) =
+            make_float4(v[c].x / rms * k[c].x, v[c].y / rms * k[c].y, v[c].z / rms * k[c].z,
+                        v[c].w / rms * k[c].w);
+    }
+    return;
+  }
+  pdl_launch_dependents();
+  pdl_wait();
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) ss += xr[i] * xr[i];
   ss = block_sum(ss, red);
   float rms = sqrtf(ss / (float)hidden + eps);
@@ -95,6 +127,8 @@ __global__ void __launch_bounds__(256)
 
 __global__ void residual_add_kernel(float* __restrict__ h, const float* __restrict__ p,
                                     int64_t n) {
+  pdl_launch_dependents();
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) h[i] = h[i] + p[i];
 }
@@ -148,7 +182,13 @@ __global__ void greedy_token_kernel(const float* __restrict__ logits, uint32_t* 
 
 int32_t launch_rmsnorm(kanso_cuda_ctx* ctx, const float* x, const float* w, float* out,
                        int64_t rows, int64_t hidden, float eps) {
-  rmsnorm_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(x, w, out, (int)hidden, eps);
+  // 2048 columns, two rows: 6.4 us a float at a time, twice over the row and launched plainly, 2.4 so
+  const bool vec = hidden % 4 == 0 && hidden <= RMS_KEEP * 1024 && aligned16(x) && aligned16(w) &&
+                   aligned16(out);
+  const cudaError_t e =
+      launch_dependent(ctx, vec ? rmsnorm_kernel<true> : rmsnorm_kernel<false>, dim3((unsigned)rows),
+                       dim3(256), 0, x, w, out, (int)hidden, eps);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "rmsnorm launch");
   return after_launch(ctx, "rmsnorm");
 }
 
@@ -178,7 +218,9 @@ int32_t launch_silu_mul(kanso_cuda_ctx* ctx, const float* g, const float* u, flo
 }
 
 int32_t launch_residual_add(kanso_cuda_ctx* ctx, float* h, const float* p, int64_t n) {
-  residual_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(h, p, n);
+  const cudaError_t e = launch_dependent(ctx, residual_add_kernel, dim3((unsigned)((n + 255) / 256)),
+                                         dim3(256), 0, h, p, n);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "residual_add launch");
   return after_launch(ctx, "residual_add");
 }
 

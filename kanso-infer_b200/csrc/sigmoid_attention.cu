@@ -428,10 +428,24 @@ __global__ void __launch_bounds__(SG_THREADS) sigmoid_group_kernel(const RowsArg
     auto squares = [&](int first, int n) {
       float acc = 0.f;
       if (four) {
+        constexpr int AT_ONCE = 4;  // columns' loads of all parts that are on their way together
+        for (int i0 = tid * 4; i0 < n; i0 += SG_THREADS * 4 * AT_ONCE) {
+          float4 v[AT_ONCE];
+#pragma unroll
+          for (int c = 0; c < AT_ONCE; ++c) v[c] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-        for (int i = tid * 4; i < n; i += SG_THREADS * 4) {
-          const float4 v = value4(first + i);
-          acc += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+          for (int r = 0; r < p.s.parts; ++r)
+#pragma unroll
+            for (int c = 0; c < AT_ONCE; ++c) {
+              const int i = i0 + c * SG_THREADS * 4;
+              if (i >= n) continue;
+              const float4 u =
+                  *reinterpret_cast<const float4*>(src + r * p.s.part_stride + first + i);
+              v[c].x += u.x, v[c].y += u.y, v[c].z += u.z, v[c].w += u.w;
+            }
+#pragma unroll
+          for (int c = 0; c < AT_ONCE; ++c)
+            acc += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
         }
       } else {
         for (int i = tid; i < n; i += SG_THREADS) {
