@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(PD_NT, HD == 64 ? 3 : 2)
   auto load = [&](uint32_t i, uint32_t p) {
     if (i && i % 32 == 0) blocks = tile_block(i + lane);
     const uint32_t phys = __shfl_sync(0xFFFFFFFFu, blocks, i & 31);
-    if (elect_one()) {
+    if (lane == 0) {
       uint64_t* bar = &s_full[warp][p % SLOTS];
       uint8_t* dst = ring + p % SLOTS * TB;
       const uint8_t* rec = a.g.pool + a.g.rec_offset(a.layer, phys, kvh);
