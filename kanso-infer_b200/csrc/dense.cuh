@@ -240,6 +240,7 @@ struct ResidualSource {
   const uint32_t* slot = nullptr;  // [T*top]: where the output of a (row, choice) pair lies
   const float* weight = nullptr;   // [T*top]
   int top = 0;
+  bool own_norm = false;  // see QkvSource
 };
 // y[t] = the weighted sum of a row's expert outputs, without the residual step
 int32_t launch_expert_sum(kanso_cuda_ctx* ctx, const float* ye, const uint32_t* slot,
@@ -260,12 +261,16 @@ struct QkvSource {
   const float* q_norm = nullptr;
   const float* k_norm = nullptr;
   float eps = 0.f;
+  // The norms' weights are a model's, uploaded before its first step, and are read while the kernel in
+  // front still runs. A caller's arrays may be what that kernel writes.
+  bool own_norm = false;
 };
 int32_t launch_qk_norm_store(kanso_cuda_ctx* ctx, int32_t compute, const QkvSource& s,
                              const KvDenseLayer& kv, uint32_t H, const RowMap& map, void* q_out,
                              int64_t T);
 // Router (f32 weights, bias or nullptr) and choice: the experts and their weights per (row, place),
-// rows per expert in counts (cleared by the caller), place within the expert in slot
+// rows per expert in counts (cleared by the caller), place within the expert in slot. The router is read
+// before the wait for the kernel in front: a model's, or with a plain launch between it and its writer.
 int32_t launch_route(kanso_cuda_ctx* ctx, const float* x, int64_t width, const DenseMat& router,
                      const float* bias, uint32_t top, RouteWeights form, uint32_t* sel, float* weight, uint32_t* counts, uint32_t* slot,
                      int64_t T);
@@ -507,8 +512,9 @@ size_t mlstm_chunk_bytes(uint32_t heads, uint32_t dim, uint32_t vdim, int64_t T)
 int32_t launch_mlstm_chunks(kanso_cuda_ctx* ctx, const MlstmArgs& a, uint32_t n, uint32_t max_rows,
                             void* mem, int64_t T);
 // out[t] = each head of o over its own root mean square, times w, times sigmoid(gate), in the
-// products' element type; the gate lies in the projections' rows.
+// products' element type; the gate lies in the projections' rows. own_norm: as in QkvSource.
 int32_t launch_head_norm_gate(kanso_cuda_ctx* ctx, int32_t compute, const MlstmArgs& a,
-                              const float* w, float eps, void* out, int64_t out_ld, int64_t T);
+                              const float* w, float eps, void* out, int64_t out_ld, int64_t T,
+                              bool own_norm);
 
 }  // namespace kanso

@@ -82,17 +82,22 @@ __global__ void __launch_bounds__(DR_THREADS)
   float ss = 0.f;
   if (four && width <= DR_KEEP * DR_THREADS * 4) {
     // A thread keeps its columns between the passes and asks for everything at once: what a row takes is
-    // the latency of its loads, and the norm's weights are there before the wait. 2048 rows of 2048 17 us and
-    // 16 so (at their bytes where four experts are added), eight rows 4.8 and 3.5.
+    // the latency of its loads, and a model's norm weights are there before the wait. 2048 rows of 2048 17 us
+    // and 16 so (at their bytes where four experts are added), eight rows 4.8 and 3.5.
     float4 y[DR_KEEP], r[DR_KEEP], k[DR_KEEP];
+    auto norm_weights = [&] {
 #pragma unroll
-    for (int c = 0; c < DR_KEEP; ++c) {
-      const int i = (threadIdx.x + c * DR_THREADS) * 4;
-      y[c] = r[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < width) k[c] = *reinterpret_cast<const float4*>(w + i);
-    }
+      for (int c = 0; c < DR_KEEP; ++c) {
+        const int i = (threadIdx.x + c * DR_THREADS) * 4;
+        if (i < width) k[c] = *reinterpret_cast<const float4*>(w + i);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < DR_KEEP; ++c) y[c] = r[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (s.own_norm) norm_weights();
     pdl_launch_dependents();
     pdl_wait();
+    if (!s.own_norm) norm_weights();
 #pragma unroll
     for (int c = 0; c < DR_KEEP; ++c) {
       const int i = (threadIdx.x + c * DR_THREADS) * 4;
@@ -261,18 +266,21 @@ __global__ void __launch_bounds__(DR_THREADS)
   const int64_t width = nq + nk + nv;
   const float* src = s.qkv + t * width;
   const bool vec = D % 8 == 0 && DV % 8 == 0 && s.part_stride % 4 == 0;
-  // a thread keeps its columns; their norms' weights are there before the wait
+  // a thread keeps its columns; a model's norm weights are there before the wait
   const bool keep = vec && width <= QK_KEEP * DR_THREADS * 4;
   float4 val[QK_KEEP], nw[QK_KEEP];
-  if (keep)
+  auto norm_weights = [&] {
 #pragma unroll
     for (int c = 0; c < QK_KEEP; ++c) {
       const int i = (threadIdx.x + c * DR_THREADS) * 4;
       if (i < nq + nk)
         nw[c] = *reinterpret_cast<const float4*>(i < nq ? s.q_norm + i : s.k_norm + i - nq);
     }
+  };
+  if (keep && s.own_norm) norm_weights();
   pdl_launch_dependents();
   pdl_wait();
+  if (keep && !s.own_norm) norm_weights();
   if (keep)
 #pragma unroll
     for (int c = 0; c < QK_KEEP; ++c) {
@@ -721,7 +729,7 @@ __global__ void __launch_bounds__(HN_THREADS)
     head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate,
                           int64_t gate_ld, int parts, int64_t part_stride, int heads, int hd,
                           const float* __restrict__ w, float eps, E* __restrict__ out,
-                          int64_t out_ld) {
+                          int64_t out_ld, bool own_norm) {
   __shared__ float red[32];
   const int h = blockIdx.x, n = heads * hd;
   const int64_t t = blockIdx.y;
@@ -733,9 +741,10 @@ __global__ void __launch_bounds__(HN_THREADS)
   const bool own = at < hd;  // a thread's columns of a head that has no more than four for each
   const bool once = hd % 4 == 0 && hd <= HN_THREADS * 4;
   float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (once && own) k4 = *reinterpret_cast<const float4*>(w + at);
+  if (own_norm && once && own) k4 = *reinterpret_cast<const float4*>(w + at);
   pdl_launch_dependents();
   pdl_wait();
+  if (!own_norm && once && own) k4 = *reinterpret_cast<const float4*>(w + at);
   if (hd % 4 == 0 && gate_ld % 4 == 0 && part_stride % 4 == 0 &&
       ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
       out_ld % 4 == 0 && once) {
@@ -935,7 +944,8 @@ int32_t launch_latent_gather(kanso_cuda_ctx* ctx, const LatentAttn& a, const KvD
 }
 
 int32_t launch_head_norm_gate(kanso_cuda_ctx* ctx, int32_t compute, const MlstmArgs& a,
-                              const float* w, float eps, void* out, int64_t out_ld, int64_t T) {
+                              const float* w, float eps, void* out, int64_t out_ld, int64_t T,
+                              bool own_norm) {
   const int H = a.heads, V = a.vdim;
   const float* gate = a.y + (int64_t)H * (2 * a.dim + V);
   const dim3 grid((unsigned)H, (unsigned)T);
@@ -943,10 +953,10 @@ int32_t launch_head_norm_gate(kanso_cuda_ctx* ctx, int32_t compute, const MlstmA
       compute == KANSO_COMPUTE_BF16
           ? launch_dependent(ctx, head_norm_gate_kernel<bf16>, grid, dim3(HN_THREADS), 0, a.out,
                              gate, a.width(), a.parts, a.part_stride, H, V, w, eps, (bf16*)out,
-                             out_ld)
+                             out_ld, own_norm)
           : launch_dependent(ctx, head_norm_gate_kernel<float>, grid, dim3(HN_THREADS), 0, a.out,
                              gate, a.width(), a.parts, a.part_stride, H, V, w, eps, (float*)out,
-                             out_ld);
+                             out_ld, own_norm);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "head_norm_gate");
   return after_launch(ctx, "head_norm_gate");
 }

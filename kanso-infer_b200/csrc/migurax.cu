@@ -430,6 +430,7 @@ int32_t MiguraxModel::run_rows(kanso_cuda_kv* kv, const DenseStep& s, float* log
     g->form = Residual::kAddNorm;
     if (out && !fold) {
       ResidualSource r;
+      r.own_norm = true;
       r.y = out;
       const int32_t e = launch_residual_norm(ctx, compute, cur, W, r, out_norm, cfg.eps, cfg.alpha,
                                              Residual::kAddNorm, nullptr, 0, T);
@@ -678,7 +679,8 @@ int32_t MiguraxModel::memory_tiles(kanso_cuda_kv* kv, size_t l, const DenseStep&
     b.portions = s.portions + s.n_short;
     if ((st = launch_mlstm_chunks(ctx, b, s.n_long, s.max_long_rows, chunk_mem, s.T))) return st;
   }
-  return launch_head_norm_gate(ctx, compute, a, ly.head_norm, cfg.eps, ao, ly.o.ld, s.T);
+  return launch_head_norm_gate(ctx, compute, a, ly.head_norm, cfg.eps, ao, ly.o.ld, s.T,
+                               true);
 }
 
 int32_t MiguraxModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* logits_dev) {
@@ -701,6 +703,7 @@ int32_t MiguraxModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
     if ((st = launch_gemm(ctx, compute, ly.o, ao, oy, W, rows, max_splits, &splits, T * W)))
       return st;
     ResidualSource r;
+    r.own_norm = true;
     r.y = oy;
     r.parts = splits;
     r.part_stride = T * W;
@@ -711,6 +714,7 @@ int32_t MiguraxModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
     GemmOut up_out;
     up_out.relu2 = up_out.elem = true;
     r = ResidualSource();
+    r.own_norm = true;
     if (sp.experts) {
       uint32_t* cnt = counts + l * count_step;
       GemmRows er;

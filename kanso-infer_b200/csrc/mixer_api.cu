@@ -236,7 +236,8 @@ int32_t kanso_cuda_head_norm_gate(kanso_cuda_ctx* ctx, const float* o, const flo
   a.vdim = vdim;
   a.y = y;
   a.out = const_cast<float*>(o);
-  return launch_head_norm_gate(ctx, KANSO_COMPUTE_F32, a, w, eps, out, (int64_t)heads * vdim, T);
+  return launch_head_norm_gate(ctx, KANSO_COMPUTE_F32, a, w, eps, out, (int64_t)heads * vdim, T,
+                               false);
 }
 
 }  // extern "C"

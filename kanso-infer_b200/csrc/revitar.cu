@@ -271,6 +271,7 @@ int32_t RevitarModel::run_rows(kanso_cuda_kv* kv, const DenseStep& s, float* log
     g->mult = cfg.mult;
     if (y && !fold) {
       ResidualSource r;
+      r.own_norm = true;
       r.y = y;
       const int32_t e = launch_residual_norm(ctx, compute, cur, W, r, y_norm, cfg.eps, cfg.mult,
                                              Residual::kAdd, nullptr, 0, T);
@@ -294,6 +295,7 @@ int32_t RevitarModel::run_rows(kanso_cuda_kv* kv, const DenseStep& s, float* log
     if ((st = source(&g))) return st;
     if ((st = launch_gemv(ctx, compute, ly.qkv, g, qkv, ly.qkv.rows, T))) return st;
     QkvSource src;
+    src.own_norm = true;
     src.qkv = qkv;
     src.q_norm = ly.q_norm;
     src.k_norm = ly.k_norm;
@@ -339,6 +341,7 @@ int32_t RevitarModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
     const RevLayer& ly = layers[l];
     const RevLayerSpec& sp = cfg.layers[l];
     QkvSource src;
+    src.own_norm = true;
     src.qkv = qkv;
     src.part_stride = T * ly.qkv.rows;
     src.q_norm = ly.q_norm;
@@ -351,6 +354,7 @@ int32_t RevitarModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
     if ((st = launch_gemm(ctx, compute, ly.o, ao, oy, W, rows, max_splits, &splits, T * W)))
       return st;
     ResidualSource r;
+    r.own_norm = true;
     r.y = oy;
     r.parts = splits;
     r.part_stride = T * W;
@@ -371,6 +375,7 @@ int32_t RevitarModel::run_tiles(kanso_cuda_kv* kv, const DenseStep& s, float* lo
     if ((st = launch_gemm_gate_up(ctx, compute, ly.gate, ly.up, xs, act, ly.down.ld, er))) return st;
     if ((st = launch_gemm(ctx, compute, ly.down, act, ye, W, er, 1, &splits, 0))) return st;
     r = ResidualSource();
+    r.own_norm = true;
     r.y = ye;
     r.slot = slot;
     r.weight = wgt;

@@ -1,0 +1,111 @@
+"""GPU: with KANSO_OPT_OVERLAP_WEIGHT_PREFETCH on, calls read the caller's arrays only once the library
+calls in front have written them. The option's promise is about the weight blocks of matmul calls alone.
+
+A long addition keeps the stream busy; a short one behind it writes the array in question and lets its
+dependents start at once, so that a read before the wait for it finds the old values.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+import plain_migurax as plain
+from conftest import rel_err
+from test_migurax_gpu import dev, f32, f64, guarded, unguard
+from test_revitar_gpu import u32, up8
+
+pytestmark = pytest.mark.gpu
+BUSY = 1 << 24  # elements of the long addition
+
+
+@pytest.fixture(scope="module")
+def eager(kb, torch_cuda):
+    """A context with the option on, and a function that has an array written late."""
+    torch = torch_cuda
+    ctx = kb.Context(0, torch.cuda.current_stream())
+    ctx.set_option(kb.OPT_OVERLAP_WEIGHT_PREFETCH, 1)
+    big, one = torch.zeros(BUSY, device="cuda"), torch.ones(BUSY, device="cuda")
+
+    def late(values):
+        """A zeroed array of four-byte words (`values`' kind) that the stream will have filled."""
+        words = dev(torch, values) if values.dtype == np.float32 else u32(torch, values)
+        out = torch.zeros_like(words)
+        torch.cuda.synchronize()
+        ctx.call("kanso_cuda_residual_add", big.data_ptr(), one.data_ptr(), BUSY)
+        # 0 + x is x, also where the words of small integers are read as (subnormal) floats
+        ctx.call("kanso_cuda_residual_add", out.data_ptr(), words.data_ptr(), words.numel())
+        return out, words
+
+    yield ctx, late
+    ctx.close()
+
+
+@pytest.mark.parametrize("width", [64, 2048, 2052, 50])
+@pytest.mark.parametrize("after", [0, 1])
+def test_residual_norm(eager, torch_cuda, width, after):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(width))
+    x, y, w = (f32(rng.standard_normal(s)) for s in ((7, width), (7, width), width))
+    xd, yd = guarded(torch, 7, width), dev(torch, y)
+    xd[:7] = dev(torch, x)
+    wd, keep = late(w)
+    ctx.call("kanso_cuda_residual_norm", xd.data_ptr(), yd.data_ptr(), wd.data_ptr(), 1e-6, 1.7,
+             after, 7, width)
+    ref = (plain.rms_norm(1.7 * f64(x) + y, f64(w), 1e-6) if after else
+           x + 1.7 * plain.rms_norm(f64(y), f64(w), 1e-6))
+    assert rel_err(unguard(ctx, xd), ref) <= 1e-6
+
+
+@pytest.mark.parametrize("H, G, D, DV", [(6, 2, 24, 16), (6, 2, 20, 12), (16, 4, 128, 128),
+                                         (24, 8, 128, 128)])
+@pytest.mark.parametrize("which", ["q", "k"])
+def test_qk_norm_store(kb, eager, torch_cuda, H, G, D, DV, which):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(H * D))
+    T, bs, eps, ld, one = 5, 4, 0.3, up8(D), lambda v: np.array([v], np.uint32)
+    qkv = f32(rng.standard_normal((T, H * D + G * D + G * DV)))
+    qn, kn = f32(rng.standard_normal(H * D)), f32(rng.standard_normal(G * D))
+    pool = kb.KvPool.dense(ctx, one(G), one(D), one(DV), 4, bs, kb.KV_F32)
+    q_out = guarded(torch, T, H * ld)
+    src = dev(torch, qkv)
+    pos, seq, tab = u32(torch, np.arange(T)), u32(torch, np.zeros(T)), u32(torch, [2, 1, 0, 3])
+    norms = [dev(torch, qn), dev(torch, kn)]
+    at = "qk".index(which)
+    norms[at], keep = late((qn, kn)[at])
+    ctx.call("kanso_cuda_qk_norm_store", pool.h, 0, src.data_ptr(), norms[0].data_ptr(),
+             norms[1].data_ptr(), eps, H, pos.data_ptr(), seq.data_ptr(), tab.data_ptr(), 4, T,
+             q_out.data_ptr())
+    ref = plain.rms_norm(f64(qkv[:, :H * D]), f64(qn), eps).reshape(T, H, D)
+    assert rel_err(unguard(ctx, q_out).reshape(T, H, ld)[:, :, :D], ref) <= 1e-6
+    if which == "k":
+        # the stored keys, seen through the scores of queries that equal them (one visible key, no cap)
+        q = np.zeros((1, H, ld), np.float32)
+        k = plain.rms_norm(f64(qkv[:, H * D:H * D + G * D]), f64(kn), eps).reshape(T, G, D)[0]
+        q[0, :, :D] = np.repeat(k, H // G, axis=0)
+        out = guarded(torch, 1, H * DV)
+        z = np.zeros(H, np.float32)
+        p = kb.SigmoidAttentionParams(1, H, 4, 1, D ** -0.5, 0.0, z.ctypes.data, z.ctypes.data,
+                                      z.ctypes.data)
+        qd = dev(torch, q)
+        ctx.call("kanso_cuda_sigmoid_attention", pool.h, 0, qd.data_ptr(), pos.data_ptr(),
+                 seq.data_ptr(), tab.data_ptr(), out.data_ptr(), ctypes.byref(p), 1)
+        score = np.repeat((k * k).sum(1), H // G) * D ** -0.5
+        v = f64(qkv[0, H * D + G * D:]).reshape(G, DV)
+        want = np.repeat(v, H // G, axis=0) / (1 + np.exp(-score))[:, None]
+        assert rel_err(unguard(ctx, out).reshape(H, DV), want) <= 5e-6
+    pool.destroy()
+
+
+@pytest.mark.parametrize("V", [37, 64, 512, 516])
+def test_head_norm_gate(eager, torch_cuda, V):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(V))
+    T, H, D, eps = 5, 4, 4, 0.2
+    o, w = f32(rng.standard_normal((T, H, V))), f32(rng.standard_normal(H * V))
+    y = f32(rng.standard_normal((T, H * (2 * D + 2 * V + 2))) * 3)
+    out, od, yd = guarded(torch, T, H * V), dev(torch, o), dev(torch, y)
+    wd, keep = late(w)
+    ctx.call("kanso_cuda_head_norm_gate", od.data_ptr(), yd.data_ptr(), wd.data_ptr(), eps,
+             out.data_ptr(), T, H, D, V)
+    gate = y[:, H * (2 * D + V):H * (2 * D + 2 * V)]
+    assert rel_err(unguard(ctx, out), plain.head_norm_gate(f64(o), f64(gate), f64(w), eps)) <= 2e-6
