@@ -737,17 +737,20 @@ __global__ void __launch_bounds__(HN_THREADS)
   E* dst = out + t * out_ld + h * hd;
   w += h * hd;
   float ss = 0.f;
+  // four columns at a time where every array lets us
+  const bool four = hd % 4 == 0 && gate_ld % 4 == 0 && part_stride % 4 == 0 && out_ld % 4 == 0 &&
+                    ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(gate) |
+                      reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) &
+                     15u) == 0;
   const int at = threadIdx.x * 4;
   const bool own = at < hd;  // a thread's columns of a head that has no more than four for each
-  const bool once = hd % 4 == 0 && hd <= HN_THREADS * 4;
+  const bool once = four && hd <= HN_THREADS * 4;
   float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f);
   if (own_norm && once && own) k4 = *reinterpret_cast<const float4*>(w + at);
   pdl_launch_dependents();
   pdl_wait();
   if (!own_norm && once && own) k4 = *reinterpret_cast<const float4*>(w + at);
-  if (hd % 4 == 0 && gate_ld % 4 == 0 && part_stride % 4 == 0 &&
-      ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
-      out_ld % 4 == 0 && once) {
+  if (once) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f), z = v;
     if (own) {
       v = *reinterpret_cast<const float4*>(x + at);
@@ -759,9 +762,7 @@ __global__ void __launch_bounds__(HN_THREADS)
     if (own)
       store4(dst + at, v.x * inv * k4.x / (1.0f + expf(-z.x)), v.y * inv * k4.y / (1.0f + expf(-z.y)),
              v.z * inv * k4.z / (1.0f + expf(-z.z)), v.w * inv * k4.w / (1.0f + expf(-z.w)));
-  } else if (hd % 4 == 0 && gate_ld % 4 == 0 && part_stride % 4 == 0 &&
-             ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
-             out_ld % 4 == 0) {
+  } else if (four) {
     for (int i = threadIdx.x * 4; i < hd; i += HN_THREADS * 4)
       ss += sum_sq4(*reinterpret_cast<const float4*>(x + i));
     ss = block_sum(ss, red);

@@ -475,6 +475,33 @@ def test_head_norm_and_gate(ctx, torch_cuda):
     assert rel_err(unguard(ctx, out), plain.head_norm_gate(f64(o), f64(gate), f64(w), eps)) <= 2e-6
 
 
+@pytest.mark.parametrize("off", ["", "o", "y", "w", "out", "o w", "y w", "o y w out"])
+@pytest.mark.parametrize("V", [64, 512, 516, 37])
+def test_head_norm_and_gate_off_16_bytes(ctx, torch_cuda, V, off):
+    """Arrays that start on any four bytes, alone and together."""
+    torch = torch_cuda
+    rng = np.random.Generator(np.random.PCG64(V))
+    T, H, D, eps = 3, 4, 4, 0.2
+    o, w = f32(rng.standard_normal((T, H, V))), f32(rng.standard_normal(H * V))
+    y = f32(rng.standard_normal((T, H * (2 * D + 2 * V + 2))) * 3)
+
+    def place(name, values):
+        buf = torch.full((values.size + 8,), float("nan"), device="cuda")
+        at = 1 if name in off.split() else 0
+        buf[at:at + values.size] = dev(torch, values).flatten()
+        return buf[at:], buf
+
+    (od, _), (yd, _), (wd, _) = place("o", o), place("y", y), place("w", w)
+    out, whole = place("out", np.zeros((T, H * V), np.float32))
+    ctx.call("kanso_cuda_head_norm_gate", od.data_ptr(), yd.data_ptr(), wd.data_ptr(), eps,
+             out.data_ptr(), T, H, D, V)
+    ctx.sync()
+    gate = y[:, H * (2 * D + V):H * (2 * D + 2 * V)]
+    got = out[:T * H * V].cpu().numpy().reshape(T, -1)
+    assert rel_err(got, plain.head_norm_gate(f64(o), f64(gate), f64(w), eps)) <= 2e-6
+    assert int(torch.isnan(whole).sum()) == 8  # nothing around the results
+
+
 # ----------------------------------------------------------------------- whole models ----
 class MiguraxCase(Case):
     models, weights, plain_class = MODELS, staticmethod(weights), plain
