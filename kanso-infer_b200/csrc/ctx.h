@@ -104,6 +104,20 @@ inline cudaError_t launch_dependent(kanso_cuda_ctx* ctx, void (*kern)(KArgs...),
   return cudaLaunchKernelEx(&lc, kern, std::forward<Args>(args)...);
 }
 
+// Launches inside a scope of this kind carry no such attribute: for calls of their own on kernels that read
+// positions, tables and lengths before the wait. A model's step uploads those before its first kernel; a
+// caller of a single mechanism may have them written by the kernel in front.
+struct PlainLaunches {
+  kanso_cuda_ctx* ctx;
+  const bool was;
+  explicit PlainLaunches(kanso_cuda_ctx* c) : ctx(c), was(c->overlap_weight_prefetch) {
+    ctx->overlap_weight_prefetch = false;
+  }
+  ~PlainLaunches() { ctx->overlap_weight_prefetch = was; }
+  PlainLaunches(const PlainLaunches&) = delete;
+  PlainLaunches& operator=(const PlainLaunches&) = delete;
+};
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 #define KANSO_CUDA_TRY(ctx, expr, what)                          \

@@ -33,6 +33,7 @@ int32_t kanso_cuda_sigmoid_attention(kanso_cuda_ctx* ctx, const kanso_cuda_kv* k
                                      float* out, const kanso_sigmoid_attention_params* p,
                                      int32_t path) {
   if (!ctx) return fail(nullptr, KANSO_ERR_CONFIG, "sigmoid_attention: ctx is NULL");
+  const PlainLaunches plain(ctx);
   if (!kv || !p || !q || !positions || !block_tables || !out)
     return fail(ctx, KANSO_ERR_SHAPE, "sigmoid_attention: NULL argument");
   if (!aligned16(q) || !aligned16(out))

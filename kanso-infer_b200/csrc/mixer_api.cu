@@ -86,6 +86,7 @@ int32_t kanso_cuda_latent_store(kanso_cuda_ctx* ctx, kanso_cuda_kv* kv, uint32_t
                                 const uint32_t* row_seq, const uint32_t* block_tables,
                                 const kanso_latent_attention_params* p, void* cq) {
   if (!ctx) return fail(nullptr, KANSO_ERR_CONFIG, "latent_store: ctx is NULL");
+  const PlainLaunches plain(ctx);
   if (!kv || !down || !q_rank || !q_norm || !c_norm || !positions || !block_tables || !p || !cq)
     return fail(ctx, KANSO_ERR_SHAPE, "latent_store: NULL argument");
   int32_t st = check_latent_pool(ctx, kv, layer, p);
@@ -111,6 +112,7 @@ int32_t kanso_cuda_latent_attention(kanso_cuda_ctx* ctx, const kanso_cuda_kv* kv
                                     float* out, const kanso_latent_attention_params* p,
                                     int32_t path) {
   if (!ctx) return fail(nullptr, KANSO_ERR_CONFIG, "latent_attention: ctx is NULL");
+  const PlainLaunches plain(ctx);
   if (!kv || !q_lat || !q || !positions || !block_tables || !out || !p || !p->sink)
     return fail(ctx, KANSO_ERR_SHAPE, "latent_attention: NULL argument");
   if (!aligned16(q_lat) || !aligned16(q) || !aligned16(out))

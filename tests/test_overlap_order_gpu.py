@@ -10,12 +10,14 @@ import numpy as np
 import pytest
 
 import plain_migurax as plain
+import plain_revitar
 from conftest import rel_err
-from test_migurax_gpu import dev, f32, f64, guarded, unguard
-from test_revitar_gpu import u32, up8
+from revitar_cases import to_bf16
+from test_migurax_gpu import LatentCase, dev, f32, f64, guarded, unguard
+from test_revitar_gpu import BF16, F32, PagedCase, to_dev, u32, unit_rows, up8
 
 pytestmark = pytest.mark.gpu
-BUSY = 1 << 24  # elements of the long addition
+BUSY = 1 << 28  # elements of the long addition: half a millisecond
 
 
 @pytest.fixture(scope="module")
@@ -109,3 +111,76 @@ def test_head_norm_gate(eager, torch_cuda, V):
              out.data_ptr(), T, H, D, V)
     gate = y[:, H * (2 * D + V):H * (2 * D + 2 * V)]
     assert rel_err(unguard(ctx, out), plain.head_norm_gate(f64(o), f64(gate), f64(w), eps)) <= 2e-6
+
+
+@pytest.mark.parametrize("compute", [F32, BF16])
+@pytest.mark.parametrize("which", ["positions", "tables"])
+def test_sigmoid_attention(kb, eager, torch_cuda, compute, which):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(3))
+    n, H, G, D, DV, T, window = 300, 6, 3, 64, 64, 5, 100
+    k, v = unit_rows(rng.standard_normal((n, G, D))), to_bf16(rng.standard_normal((n, G, DV)))
+    q, at = to_bf16(rng.standard_normal((T, H, D))), np.array([299, 40, 7, 160, 220])
+    case = PagedCase(kb, ctx, torch, rng, k, v, 16, compute, H)
+    z = np.zeros(H, np.float32)
+    p = kb.SigmoidAttentionParams(T, H, case.nb, window, D ** -0.5, 5.0, z.ctypes.data, z.ctypes.data,
+                                  z.ctypes.data)
+    qd, out, seq = to_dev(torch, q, compute), guarded(torch, T, H * DV), u32(torch, np.zeros(T))
+    pos, tab = u32(torch, at), case.tables
+    if which == "positions":
+        pos, keep = late(at.astype(np.uint32))
+    else:
+        tab, keep = late(case.table)
+    ctx.call("kanso_cuda_sigmoid_attention", case.pool.h, 0, qd.data_ptr(), pos.data_ptr(),
+             seq.data_ptr(), tab.data_ptr(), out.data_ptr(), ctypes.byref(p), 1)
+    kk = f64(k if compute == F32 else to_bf16(k))
+    ref = plain_revitar.attention_core(f64(q), kk, f64(v), at, np.arange(n), D ** -0.5, 5.0, f64(z),
+                                       f64(z), f64(z), window)
+    assert rel_err(unguard(ctx, out).reshape(T, H, DV), ref) <= (5e-6 if compute == F32 else 1e-2)
+    case.pool.destroy()
+
+
+@pytest.mark.parametrize("compute", [F32, BF16])
+@pytest.mark.parametrize("which", ["positions", "tables"])
+def test_latent_store_and_attention(kb, eager, torch_cuda, compute, which):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(4))
+    n, H, rank, rot, dim, T, bs, base = 300, 3, 64, 16, 7, 4, 16, 500.0
+    raw, c_norm = rng.standard_normal((n, rank + rot)), f32(rng.uniform(0.5, 1.5, rank))
+    case = LatentCase(kb, ctx, torch, rng, raw, c_norm, rank, base, bs, compute)
+    tol = 1e-5 if compute == F32 else 2e-2
+
+    def one_late(at):
+        """Positions and tables, one of them written late."""
+        pos, tab = u32(torch, at), case.tables
+        if which == "positions":
+            pos, keep = late(at.astype(np.uint32))
+        else:
+            tab, keep = late(case.tables.cpu().numpy().astype(np.uint32))
+        return pos, tab, keep
+
+    # the last rows once more, with other values
+    at = np.arange(n - T, n)
+    raw[at] = rng.standard_normal((T, rank + rot))
+    down, qn = f32(np.concatenate([rng.standard_normal((T, 13)), raw[at]], 1)), np.ones(13, np.float32)
+    arrays, seq = [dev(torch, a) for a in (down, qn, c_norm)], u32(torch, np.zeros(T))
+    cq = torch.zeros(T * 32, device="cuda")
+    p = case.params(T, 1, 1, 1.0, None)
+    pos, tab, keep = one_late(at)
+    ctx.call("kanso_cuda_latent_store", case.pool.h, 0, arrays[0].data_ptr(), 13,
+             arrays[1].data_ptr(), arrays[2].data_ptr(), 1e-5, pos.data_ptr(), seq.data_ptr(),
+             tab.data_ptr(), ctypes.byref(p), cq.data_ptr())
+    case.c = plain.rms_norm(f64(f32(raw[:, :rank])), f64(c_norm), 1e-5)
+    case.k_rot = plain.rotate(f64(f32(raw[:, rank:])), np.arange(n), base)
+
+    at = np.array([299, 296, 20, 150])
+    q_lat, q = rng.standard_normal((T, H, rank)) * 3, rng.standard_normal((T, H, dim + rot)) * 3
+    sink, out = f32(rng.uniform(-1, 1, H)), guarded(torch, T, H * rank)
+    ql, qq = dev(torch, q_lat), dev(torch, q)
+    p = case.params(T, H, dim, 0.1, sink)
+    pos, tab, keep = one_late(at)
+    ctx.call("kanso_cuda_latent_attention", case.pool.h, 0, ql.data_ptr(), qq.data_ptr(),
+             pos.data_ptr(), seq.data_ptr(), tab.data_ptr(), out.data_ptr(), ctypes.byref(p), 0)
+    got = unguard(ctx, out).reshape(T, H, rank)
+    assert rel_err(got, case.reference(q_lat, q, at, 0.1, sink)) <= tol
+    case.pool.destroy()
