@@ -69,7 +69,8 @@ __device__ __forceinline__ float from_elem(float v) { return v; }
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float relu_squared(float z) {
-  const float r = fmaxf(z, 0.f);
+  float r;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(z));  // a value that is none stays none
   return r * r;
 }
 

@@ -86,7 +86,6 @@ __device__ __forceinline__ void ext_rows(const GemmDenseArgs& a, const RowPlace&
                                          uint32_t tmem, int n, int64_t first, int valid) {
   const float b0 = a.bias_of(n), b1 = DUAL ? a.bias_of(n + 128) : 0.f;
   const bool in0 = n < a.n_end, in1 = DUAL && n + 128 < a.n_end, sq = a.relu2;
-  const float low = sq ? 0.f : -INFINITY;
   const int64_t ld = a.out_ld;
   out += place.shift + n;
   for (int c = 0; c < NT; c += 16) {
@@ -98,12 +97,12 @@ __device__ __forceinline__ void ext_rows(const GemmDenseArgs& a, const RowPlace&
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       if (c + j >= valid) continue;
-      const float x = fmaxf(__uint_as_float(r0[j]) + b0, low);
+      const float x = __uint_as_float(r0[j]) + b0;
       O* at = place.list ? out + place.list[first + c + j - place.first] * ld : o + j * ld;
-      if (in0) at[0] = to_elem<O>(sq ? x * x : x);
+      if (in0) at[0] = to_elem<O>(sq ? relu_squared(x) : x);
       if (DUAL) {
-        const float y = fmaxf(__uint_as_float(r1[j]) + b1, low);
-        if (in1) at[128] = to_elem<O>(sq ? y * y : y);
+        const float y = __uint_as_float(r1[j]) + b1;
+        if (in1) at[128] = to_elem<O>(sq ? relu_squared(y) : y);
       }
     }
   }

@@ -207,13 +207,13 @@ __device__ __forceinline__ bool partners_any(int bar, bool mine) {
 template <typename O>
 __device__ __forceinline__ void gp_store_ext(const GemmDenseArgs& a, const RowPlace& place, O* out,
                                              const uint32_t (&r)[16], int n, int64_t row0, int valid) {
-  const float bias = a.bias_of(n), low = a.relu2 ? 0.f : -INFINITY;
+  const float bias = a.bias_of(n);
   if (n >= a.n_end) return;
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     if (j >= valid) continue;
-    const float x = fmaxf(__uint_as_float(r[j]) + bias, low);
-    out[place.at(row0 + j, a.out_ld) + n] = to_elem<O>(a.relu2 ? x * x : x);
+    const float x = __uint_as_float(r[j]) + bias;
+    out[place.at(row0 + j, a.out_ld) + n] = to_elem<O>(a.relu2 ? relu_squared(x) : x);
   }
 }
 

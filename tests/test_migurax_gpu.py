@@ -59,6 +59,32 @@ def test_linear_with_bias_and_squared_relu(ctx, torch_cuda, compute, rows, cols)
                 assert rel_err(unguard(ctx, y), want) <= 4e-6, (T, path, relu2)
 
 
+@pytest.mark.parametrize("compute, path, T, rows", [
+    (F32, 1, 2, 50), (F32, 2, 40, 50), (BF16, 1, 2, 50), (BF16, 2, 40, 300),
+    (BF16, 2, 70, 80000),   # two tiles of weight rows for each CTA
+    (BF16, 2, 100, 14400),  # pairs of CTAs
+])
+def test_linear_keeps_what_is_no_number(ctx, torch_cuda, compute, path, T, rows):
+    """A row of x with a NaN has nothing but NaN for results, behind bias and squared ReLU too."""
+    torch = torch_cuda
+    rng = np.random.Generator(np.random.PCG64(rows))
+    cols = 800 if rows > 50000 else 72
+    w, b = to_bf16(rng.standard_normal((rows, cols))), f32(rng.standard_normal(rows) * 5)
+    x = to_bf16(rng.standard_normal((T, cols)))
+    ref = f64(x) @ f64(w).T + b
+    x[T - 1, 3] = np.nan
+    wd, bd, xd = to_dev(torch, w, compute), dev(torch, b), to_dev(torch, x, compute)
+    for relu2 in (0, 1):
+        y = torch.zeros(T, rows, device="cuda")
+        ctx.call("kanso_cuda_dense_linear_act", compute, wd.data_ptr(), xd.data_ptr(), bd.data_ptr(),
+                 relu2, y.data_ptr(), T, rows, cols, path)
+        ctx.sync()
+        got = y.cpu().numpy()
+        assert np.isnan(got[T - 1]).all()
+        want = plain.relu_squared(ref) if relu2 else ref
+        assert rel_err(got[:T - 1], want[:T - 1]) <= 4e-6
+
+
 @pytest.mark.parametrize("compute", [F32, BF16])
 @pytest.mark.parametrize("experts, top, width, ff", [(5, 2, 72, 40), (1, 1, 64, 24), (40, 7, 52, 33),
                                                      (6, 6, 200, 130), (130, 3, 128, 64)])
