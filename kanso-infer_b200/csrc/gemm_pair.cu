@@ -37,6 +37,7 @@ constexpr int GP_STAGE = 2 * GP_HALF;
 constexpr int GP_STAGES = 6;
 constexpr int GP_ACCS = 2;  // tiles whose results TMEM holds
 constexpr uint32_t GP_POLLS = 1u << 18;  // about a second: a poll that finds nothing lasts 4 us
+constexpr uint32_t GP_LAND_POLLS = 1u << 12;  // about 16 ms, for what is on its way when a CTA gives up
 constexpr size_t GP_SMEM = (size_t)GP_STAGE * GP_STAGES + 1024;
 
 // What `tiles` of n activation rows cost `pairs` pairs, in cycles per 16 columns: a wave takes the products'
@@ -157,6 +158,19 @@ __device__ __forceinline__ bool mbar_wait_pair(uint64_t* bar, uint32_t parity,
   *abort_flag = 1;
   return false;
 }
+// Until what a CTA that gives up has still on its way has landed or retired. A stage that the other CTA never
+// asked for does not complete: there the limit ends the wait, long after this CTA's own copies.
+__device__ __forceinline__ void mbar_wait_land(uint64_t* bar, uint32_t parity) {
+  mbar_wait_bounded(bar, parity, GP_LAND_POLLS);
+}
+// A word of the other CTA's shared memory, at the same place.
+__device__ __forceinline__ void store_other(volatile int* p, uint32_t rank, int v) {
+  asm volatile(
+      "{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, %1;\nst.shared::cluster.u32 [a], %2;\n}\n" ::"r"(
+          smem_u32(const_cast<int*>(p))),
+      "r"(rank ^ 1u), "r"(v)
+      : "memory");
+}
 // Copies into this CTA's shared memory whose bytes count on the even CTA's barrier.
 __device__ __forceinline__ void pair_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                              uint32_t bar) {
@@ -228,7 +242,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   __shared__ uint64_t full[GP_STAGES], empty[GP_STAGES], acc_full[GP_ACCS], acc_empty[GP_ACCS];
   __shared__ float swap[GATE_UP ? 8 : 1][2][8][32];  // what a warp hands to its partner, two chunks
   __shared__ uint32_t tmem_slot;
-  __shared__ volatile int abort_flag;
+  __shared__ volatile int abort_flag, other_issued;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const int first_tile = (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
@@ -244,7 +258,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       mbar_init(&acc_empty[i], 16);  // the result warps of both CTAs
     }
     mbar_fence_init();
-    abort_flag = 0;
+    abort_flag = other_issued = 0;
   }
   cluster_sync();
   pdl_launch_dependents();
@@ -261,10 +275,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const int max_n = gp_max_n(a, tiles, lane, step);
+  int issued = 0;  // warp 0: the stages that it has asked for
 
   if (warp == 0) {
     // ---- copies: this CTA's weight rows and its half of the activation rows ----
-    int issued = 0;
     bool ok = true;
     GpTile t;
     for (int tile = first_tile; ok && gp_tile(a, tiles, max_n, tile, lane, &t); tile += step) {
@@ -324,7 +338,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
             pair_mma(acc, ad + 2 * j, bd + 2 * j, idesc, (k > 0 || j > 0) ? 1u : 0u);
           pair_commit(&empty[s]);
         }
-        if (ok) pair_commit(&acc_full[b]);
+        if (ok)
+          pair_commit(&acc_full[b]);
+        else if (at)  // the products issued so far still read shared memory
+          mbar_wait_land(&empty[(at - 1) % GP_STAGES], ((at - 1) / GP_STAGES) & 1u);
       }
       ok = __all_sync(0xFFFFFFFFu, ok);
       at = __reduce_max_sync(0xFFFFFFFFu, at);
@@ -386,14 +403,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     }
   }
   __syncthreads();
-  // A CTA that gave up may have copies of its own on their way: they land before it ends (bounded).
-  const int failed = abort_flag != 0;
-  if (failed && threadIdx.x == 0) {
+  if (abort_flag && threadIdx.x == 0) {
     atomicOr(a.status, DEV_WAIT_TIMEOUT);
-    __nanosleep(1000000);
+    store_other(&other_issued, rank, issued);
+    store_other(&abort_flag, rank, 1);
   }
   tc_fence_before();
   cluster_sync();
+  if (abort_flag) {  // in both CTAs: one of them has given up
+    // Copies of both that are still on their way land before either ends (bounded); they count on the
+    // even CTA's barriers.
+    if (warp == 0 && rank == 0) {
+      const int last = max(issued, other_issued);
+      for (int i = max(0, last - GP_STAGES); i < last; ++i)
+        mbar_wait_land(&full[i % GP_STAGES], (uint32_t)(i / GP_STAGES) & 1u);
+    }
+    cluster_sync();
+  }
   if (warp == 2)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
