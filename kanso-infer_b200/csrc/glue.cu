@@ -9,20 +9,21 @@
 namespace kanso {
 
 // x / sqrt(mean(x^2) + eps) * w, one CTA per row (src/model.rs:653-659).
-constexpr int RMS_KEEP = 4;
-template <bool VEC>
+// VEC: rows of whole float4. KEEP: float4 of a row that a thread keeps between the passes, for rows of at most
+// KEEP * 1024 columns (0: wider ones are read twice).
+template <bool VEC, int KEEP>
 __global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                float* __restrict__ out, int hidden, float eps) {
   __shared__ float red[32];
   const float* xr = x + (int64_t)blockIdx.x * hidden;
   float ss = 0.f;
-  if (VEC) {  // hidden % 4 == 0, at most RMS_KEEP * 1024: a thread keeps its columns
+  if constexpr (KEEP > 0) {
     float* o = out + (int64_t)blockIdx.x * hidden;
-    float4 v[RMS_KEEP], k[RMS_KEEP];
+    float4 v[KEEP], k[KEEP];
     pdl_launch_dependents();
     pdl_wait();
 #pragma unroll
-    for (int c = 0; c < RMS_KEEP; ++c) {
+    for (int c = 0; c < KEEP; ++c) {
       const int i = (threadIdx.x + c * 256) * 4;
       v[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (i < hidden) {
@@ -31,11 +32,11 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restr
       }
     }
 #pragma unroll
-    for (int c = 0; c < RMS_KEEP; ++c)
+    for (int c = 0; c < KEEP; ++c)
       ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
     const float rms = sqrtf(block_sum(ss, red) / (float)hidden + eps);
 #pragma unroll
-    for (int c = 0; c < RMS_KEEP; ++c) {
+    for (int c = 0; c < KEEP; ++c) {
       const int i = (threadIdx.x + c * 256) * 4;
       if (i < hidden)
         *reinterpret_cast<float4*>(o + i) =
@@ -46,6 +47,23 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restr
   }
   pdl_launch_dependents();
   pdl_wait();
+  if constexpr (VEC) {
+    float* o = out + (int64_t)blockIdx.x * hidden;
+#pragma unroll 4
+    for (int i = threadIdx.x * 4; i < hidden; i += 1024) {
+      const float4 v = *reinterpret_cast<const float4*>(xr + i);
+      ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    }
+    const float rms = sqrtf(block_sum(ss, red) / (float)hidden + eps);
+#pragma unroll 4
+    for (int i = threadIdx.x * 4; i < hidden; i += 1024) {
+      const float4 v = *reinterpret_cast<const float4*>(xr + i);
+      const float4 k = *reinterpret_cast<const float4*>(w + i);
+      *reinterpret_cast<float4*>(o + i) =
+          make_float4(v.x / rms * k.x, v.y / rms * k.y, v.z / rms * k.z, v.w / rms * k.w);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) ss += xr[i] * xr[i];
   ss = block_sum(ss, red);
   float rms = sqrtf(ss / (float)hidden + eps);
@@ -203,12 +221,18 @@ __global__ void greedy_token_kernel(const float* __restrict__ logits, uint32_t* 
 
 int32_t launch_rmsnorm(kanso_cuda_ctx* ctx, const float* x, const float* w, float* out,
                        int64_t rows, int64_t hidden, float eps) {
-  // 2048 columns, two rows: 6.4 us a float at a time, twice over the row and launched plainly, 2.4 so
-  const bool vec = hidden % 4 == 0 && hidden <= RMS_KEEP * 1024 && aligned16(x) && aligned16(w) &&
-                   aligned16(out);
+  // us: two rows of 2048 6.4 a float at a time, twice over the row and launched plainly, 2.4 so; 512 of 5000
+  // 13.2 and 7.1. Four kept float4 take 52 registers, four CTAs an SM: rows beyond those that need one alone keep
+  // one (2048 rows of 64 5.5 us with four, 3.8 with one; 2048 of 1024 6.2 and 4.9; but 512 of 1024 2.6 and 3.0).
+  const bool vec = hidden % 4 == 0 && aligned16(x) && aligned16(w) && aligned16(out);
   const cudaError_t e =
-      launch_dependent(ctx, vec ? rmsnorm_kernel<true> : rmsnorm_kernel<false>, dim3((unsigned)rows),
-                       dim3(256), 0, x, w, out, (int)hidden, eps);
+      launch_dependent(ctx,
+                       !vec            ? rmsnorm_kernel<false, 0>
+                       : hidden > 4096 ? rmsnorm_kernel<true, 0>
+                       : hidden <= 1024 && rows > 4 * (int64_t)ctx->sm_count
+                           ? rmsnorm_kernel<true, 1>
+                           : rmsnorm_kernel<true, 4>,
+                       dim3((unsigned)rows), dim3(256), 0, x, w, out, (int)hidden, eps);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "rmsnorm launch");
   return after_launch(ctx, "rmsnorm");
 }

@@ -27,3 +27,18 @@ def test_residual_add(ctx, torch_cuda, n, offs):
     got = hb.cpu().numpy()
     assert (got[offs[0]:offs[0] + n] == h + p).all()  # one rounding: exact
     assert np.isnan(got[:offs[0]]).all() and np.isnan(got[offs[0] + n:]).all()
+
+
+@pytest.mark.parametrize("rows, hidden", [(5, h) for h in (1, 50, 64, 1000, 1024, 1028, 4096, 4100, 8192, 9001)] +
+                         [(700, 4), (700, 1024)])  # more rows than four to an SM
+@pytest.mark.parametrize("off", [None, "x", "w", "out"])
+def test_rmsnorm(ctx, oracle, torch_cuda, rows, hidden, off):
+    rng = np.random.Generator(np.random.PCG64(hidden))
+    x, w = rng.standard_normal((rows, hidden)).astype(np.float32), rng.standard_normal(hidden).astype(np.float32)
+    (_, xd), (_, wd), (ob, od) = (place(torch_cuda, a, int(off == n)) for a, n in
+                                  ((x, "x"), (w, "w"), (np.zeros_like(x), "out")))
+    ctx.rmsnorm(xd, wd, od, rows, hidden, 1e-5)
+    ctx.sync()
+    got = od.cpu().numpy()
+    assert rel_err(got[:rows * hidden].reshape(rows, -1), oracle.rmsnorm(x, w, 1e-5)) <= 2e-6
+    assert np.isnan(got[rows * hidden:]).all() and int(torch_cuda.isnan(ob).sum()) == 2 + int(off == "out")
