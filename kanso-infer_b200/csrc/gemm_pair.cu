@@ -363,7 +363,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       const RowPlace place(a, t.group);
       for (int c = half * 16; c < t.n && c < t.valid; c += 32) {
         uint32_t r0[16];
-        __syncwarp();
         tmem_ld16(acc + c, r0);
         const int64_t row0 = t.first + c;
         const int valid = t.valid - c;

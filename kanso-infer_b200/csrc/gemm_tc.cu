@@ -343,6 +343,7 @@ __device__ __forceinline__ void tc_dequant_q4_k(const uint8_t* raw_stage, int s,
 // The producers' barrier: true for all of them when one of them has seen the CTA give up.
 __device__ __forceinline__ bool producers_abort(bool mine) {
   uint32_t any;
+  __syncwarp();  // the lanes have polled one by one
   asm volatile(
       "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred.aligned q, 1, %2, p;\n"
       "selp.b32 %0, 1, 0, q;\n}\n"
