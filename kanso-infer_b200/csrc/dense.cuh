@@ -263,7 +263,8 @@ struct QkvSource {
   const float* k_norm = nullptr;
   float eps = 0.f;
   // The norms' weights are a model's, uploaded before its first step, and are read while the kernel in
-  // front still runs. A caller's arrays may be what that kernel writes.
+  // front still runs. A caller's arrays may be what that kernel writes: they are read behind the wait, and not
+  // through __restrict__ pointers, whose loads the compiler may move in front of it.
   bool own_norm = false;
 };
 int32_t launch_qk_norm_store(kanso_cuda_ctx* ctx, int32_t compute, const QkvSource& s,

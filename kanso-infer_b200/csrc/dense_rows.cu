@@ -68,10 +68,12 @@ __global__ void embed_scaled_kernel(const E* __restrict__ embed, int64_t ld,
   }
 }
 
+// w is no __restrict__ pointer: loads through one may be moved in front of the wait (and were, where the wait stands
+// behind a condition).
 template <typename E>
 __global__ void __launch_bounds__(DR_THREADS)
     residual_norm_kernel(float* __restrict__ x, int width, const ResidualSource s,
-                         const float* __restrict__ w, float eps, float mult, Residual form,
+                         const float* w, float eps, float mult, Residual form,
                          E* __restrict__ xe, int64_t xe_ld) {
   extern __shared__ __align__(16) float v[];  // [width]
   __shared__ float red[32];
@@ -728,8 +730,8 @@ template <typename E>
 __global__ void __launch_bounds__(HN_THREADS)
     head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate,
                           int64_t gate_ld, int parts, int64_t part_stride, int heads, int hd,
-                          const float* __restrict__ w, float eps, E* __restrict__ out,
-                          int64_t out_ld, bool own_norm) {
+                          const float* w, float eps, E* __restrict__ out, int64_t out_ld,
+                          bool own_norm) {
   __shared__ float red[32];
   const int h = blockIdx.x, n = heads * hd;
   const int64_t t = blockIdx.y;

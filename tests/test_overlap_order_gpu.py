@@ -184,3 +184,69 @@ def test_latent_store_and_attention(kb, eager, torch_cuda, compute, which):
     got = unguard(ctx, out).reshape(T, H, rank)
     assert rel_err(got, case.reference(q_lat, q, at, 0.1, sink)) <= tol
     case.pool.destroy()
+
+
+@pytest.mark.parametrize("rows, hidden", [(3, 50), (3, 960), (3, 2048), (3, 5000), (700, 960)])
+@pytest.mark.parametrize("which", ["x", "w"])
+def test_rmsnorm(eager, torch_cuda, rows, hidden, which):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(hidden))
+    x, w = f32(rng.standard_normal((rows, hidden))), f32(rng.standard_normal(hidden))
+    xd, wd, out = dev(torch, x), dev(torch, w), guarded(torch, rows, hidden)
+    if which == "x":
+        xd, keep = late(x)
+    else:
+        wd, keep = late(w)
+    ctx.call("kanso_cuda_rmsnorm", xd.data_ptr(), wd.data_ptr(), out.data_ptr(), rows, hidden, 1e-5)
+    assert rel_err(unguard(ctx, out), plain.rms_norm(f64(x), f64(w), 1e-5)) <= 2e-6
+
+
+@pytest.mark.parametrize("n", [100, 5000])
+@pytest.mark.parametrize("which", [0, 1])
+def test_silu_mul(eager, torch_cuda, n, which):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(n))
+    a = [f32(rng.standard_normal(n)) for _ in range(2)]
+    d, out = [dev(torch, v) for v in a], guarded(torch, 1, n)
+    d[which], keep = late(a[which])
+    ctx.call("kanso_cuda_silu_mul", d[0].data_ptr(), d[1].data_ptr(), out.data_ptr(), n)
+    g = f64(a[0])
+    assert rel_err(unguard(ctx, out)[0], g / (1 + np.exp(-g)) * a[1]) <= 1e-6
+
+
+@pytest.mark.parametrize("compute, path, T, rows", [(F32, 1, 2, 50), (F32, 2, 40, 50), (BF16, 1, 2, 50),
+                                                    (BF16, 2, 40, 300), (BF16, 2, 100, 14400)])
+def test_bias_of_a_product(eager, torch_cuda, compute, path, T, rows):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(rows))
+    w, x, b = (f32(to_bf16(rng.standard_normal(s))) for s in ((rows, 72), (T, 72), rows))
+    wd, xd, y = to_dev(torch, w, compute), to_dev(torch, x, compute), guarded(torch, T, rows)
+    bd, keep = late(b)
+    ctx.call("kanso_cuda_dense_linear_act", compute, wd.data_ptr(), xd.data_ptr(), bd.data_ptr(), 0,
+             y.data_ptr(), T, rows, 72, path)
+    assert rel_err(unguard(ctx, y), f64(x) @ f64(w).T + b) <= 4e-6
+
+
+@pytest.mark.parametrize("which", ["router", "bias"])
+@pytest.mark.parametrize("T, path", [(2, 1), (3, 2), (300, 2), (1300, 2)])
+def test_router_of_experts(eager, torch_cuda, T, path, which):
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(T))
+    experts, width, ff = 6, 64, 24
+    w = {"router": to_bf16(np.eye(experts, width) * 6), "router.b": f32(np.arange(experts) * 0.01)}
+    for e in range(experts):
+        w[f"e{e}.up"] = to_bf16(rng.standard_normal((ff, width)) * width ** -0.5)
+        w[f"e{e}.down"] = to_bf16(rng.standard_normal((width, ff)) * ff ** -0.5)
+    x = to_bf16(rng.standard_normal((T, width)))
+    x[:, :experts] = np.stack([rng.permutation(experts) for _ in range(T)])  # no close calls
+    stack = lambda n: dev(torch, np.stack([w[f"e{e}.{n}"] for e in range(experts)]))
+    xd, up, down, y = dev(torch, x), stack("up"), stack("down"), guarded(torch, T, width)
+    router, bias = dev(torch, w["router"]), dev(torch, w["router.b"])
+    if which == "router":
+        router, keep = late(f32(w["router"]))
+    else:
+        bias, keep = late(w["router.b"])
+    ctx.call("kanso_cuda_moe_relu2", F32, xd.data_ptr(), router.data_ptr(), bias.data_ptr(),
+             up.data_ptr(), down.data_ptr(), y.data_ptr(), T, width, ff, experts, 2, path)
+    ref = plain.moe(f64(x), plain.doubles(w), "", {"router": {"experts": experts, "top": 2}})
+    assert rel_err(unguard(ctx, y), ref) <= 4e-6
