@@ -70,7 +70,10 @@ __global__ void embed_scaled_kernel(const E* __restrict__ embed, int64_t ld,
 
 // w is no __restrict__ pointer: loads through one may be moved in front of the wait (and were, where the wait stands
 // behind a condition).
-template <typename E>
+// KEPT: rows of whole float4 that a thread's DR_KEEP of them cover. Wider rows have an instance of their own: with the
+// kept rows' 52 registers an SM holds four CTAs in place of five (us: 2048 x 2056 14.1, with 48 registers 12.0;
+// 2048 x 8192 56.1 and 48.8).
+template <typename E, bool KEPT>
 __global__ void __launch_bounds__(DR_THREADS)
     residual_norm_kernel(float* __restrict__ x, int width, const ResidualSource s,
                          const float* w, float eps, float mult, Residual form,
@@ -82,24 +85,20 @@ __global__ void __launch_bounds__(DR_THREADS)
   const bool after = form == Residual::kAddNorm;  // the norm is of the sum
   const bool four = width % 4 == 0 && s.part_stride % 4 == 0;
   float ss = 0.f;
-  if (four && width <= DR_KEEP * DR_THREADS * 4) {
+  if constexpr (KEPT) {
     // A thread keeps its columns between the passes and asks for everything at once: what a row takes is
     // the latency of its loads, and a model's norm weights are there before the wait. 2048 rows of 2048 17 us
     // and 16 so (at their bytes where four experts are added), eight rows 4.8 and 3.5.
     float4 y[DR_KEEP], r[DR_KEEP], k[DR_KEEP];
-    auto norm_weights = [&] {
-#pragma unroll
-      for (int c = 0; c < DR_KEEP; ++c) {
-        const int i = (threadIdx.x + c * DR_THREADS) * 4;
-        if (i < width) k[c] = *reinterpret_cast<const float4*>(w + i);
-      }
-    };
-#pragma unroll
-    for (int c = 0; c < DR_KEEP; ++c) y[c] = r[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (s.own_norm) norm_weights();
     pdl_launch_dependents();
+    if (!s.own_norm) pdl_wait();
+#pragma unroll
+    for (int c = 0; c < DR_KEEP; ++c) {
+      const int i = (threadIdx.x + c * DR_THREADS) * 4;
+      y[c] = r[c] = k[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < width) k[c] = *reinterpret_cast<const float4*>(w + i);
+    }
     pdl_wait();
-    if (!s.own_norm) norm_weights();
 #pragma unroll
     for (int c = 0; c < DR_KEEP; ++c) {
       const int i = (threadIdx.x + c * DR_THREADS) * 4;
@@ -193,20 +192,30 @@ __global__ void __launch_bounds__(DR_THREADS)
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)width + eps);
   if (four) {
-#pragma unroll 2
-    for (int i = threadIdx.x * 4; i < width; i += DR_THREADS * 4) {
-      const float4 y = *reinterpret_cast<const float4*>(v + i);
-      const float4 k = *reinterpret_cast<const float4*>(w + i);
-      float4 r;
-      if (after) {
-        r = make_float4(y.x * inv * k.x, y.y * inv * k.y, y.z * inv * k.z, y.w * inv * k.w);
-      } else {
-        r = *reinterpret_cast<const float4*>(xr + i);
-        r.x += mult * (y.x * inv * k.x), r.y += mult * (y.y * inv * k.y);
-        r.z += mult * (y.z * inv * k.z), r.w += mult * (y.w * inv * k.w);
+    constexpr int AT_ONCE = 2;  // loads of the weights and the row in front of both stores
+    for (int i0 = threadIdx.x * 4; i0 < width; i0 += AT_ONCE * DR_THREADS * 4) {
+      float4 k[AT_ONCE], r[AT_ONCE];
+#pragma unroll
+      for (int c = 0; c < AT_ONCE; ++c) {
+        const int i = i0 + c * DR_THREADS * 4;
+        k[c] = r[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < width) k[c] = *reinterpret_cast<const float4*>(w + i);
+        if (i < width && !after) r[c] = *reinterpret_cast<const float4*>(xr + i);
       }
-      *reinterpret_cast<float4*>(xr + i) = r;
-      if (xe) store4(xe + t * xe_ld + i, r.x, r.y, r.z, r.w);
+#pragma unroll
+      for (int c = 0; c < AT_ONCE; ++c) {
+        const int i = i0 + c * DR_THREADS * 4;
+        if (i >= width) continue;
+        const float4 y = *reinterpret_cast<const float4*>(v + i);
+        float4 n = make_float4(y.x * inv * k[c].x, y.y * inv * k[c].y, y.z * inv * k[c].z,
+                               y.w * inv * k[c].w);
+        if (!after) {
+          n.x = r[c].x + mult * n.x, n.y = r[c].y + mult * n.y;
+          n.z = r[c].z + mult * n.z, n.w = r[c].w + mult * n.w;
+        }
+        *reinterpret_cast<float4*>(xr + i) = n;
+        if (xe) store4(xe + t * xe_ld + i, n.x, n.y, n.z, n.w);
+      }
     }
   } else {
     for (int i = threadIdx.x; i < width; i += DR_THREADS) {
@@ -271,18 +280,16 @@ __global__ void __launch_bounds__(DR_THREADS)
   // a thread keeps its columns; a model's norm weights are there before the wait
   const bool keep = vec && width <= QK_KEEP * DR_THREADS * 4;
   float4 val[QK_KEEP], nw[QK_KEEP];
-  auto norm_weights = [&] {
+  pdl_launch_dependents();
+  if (!s.own_norm) pdl_wait();
+  if (keep)
 #pragma unroll
     for (int c = 0; c < QK_KEEP; ++c) {
       const int i = (threadIdx.x + c * DR_THREADS) * 4;
       if (i < nq + nk)
         nw[c] = *reinterpret_cast<const float4*>(i < nq ? s.q_norm + i : s.k_norm + i - nq);
     }
-  };
-  if (keep && s.own_norm) norm_weights();
-  pdl_launch_dependents();
   pdl_wait();
-  if (keep && !s.own_norm) norm_weights();
   if (keep)
 #pragma unroll
     for (int c = 0; c < QK_KEEP; ++c) {
@@ -748,10 +755,10 @@ __global__ void __launch_bounds__(HN_THREADS)
   const bool own = at < hd;  // a thread's columns of a head that has no more than four for each
   const bool once = four && hd <= HN_THREADS * 4;
   float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (own_norm && once && own) k4 = *reinterpret_cast<const float4*>(w + at);
   pdl_launch_dependents();
+  if (!own_norm) pdl_wait();
+  if (once && own) k4 = *reinterpret_cast<const float4*>(w + at);
   pdl_wait();
-  if (!own_norm && once && own) k4 = *reinterpret_cast<const float4*>(w + at);
   if (once) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f), z = v;
     if (own) {
@@ -817,11 +824,15 @@ int32_t launch_embed_scaled(kanso_cuda_ctx* ctx, int32_t compute, const void* em
 int32_t launch_residual_norm(kanso_cuda_ctx* ctx, int32_t compute, float* x, int64_t width,
                              const ResidualSource& s, const float* w, float eps, float mult,
                              Residual form, void* xe, int64_t xe_ld, int64_t T) {
-  const size_t smem = (size_t)width * 4;
+  size_t smem = (size_t)width * 4;
   if (smem > 200 * 1024)
     return fail(ctx, KANSO_ERR_UNSUPPORTED, "residual norm: width %lld", (long long)width);
-  auto kern_b = residual_norm_kernel<bf16>;
-  auto kern_f = residual_norm_kernel<float>;
+  const bool kept = width % 4 == 0 && s.part_stride % 4 == 0 && width <= DR_KEEP * DR_THREADS * 4;
+  // Wide rows that four CTAs an SM hold do not take five: with the next rows' CTAs waiting beside them the SMs' shares
+  // come out uneven (512 x 8192, call behind call: 11.6 us with five, 10.3).
+  if (!kept && T <= 4 * (int64_t)ctx->sm_count) smem = std::max<size_t>(smem, ctx->smem_per_sm / 5);
+  auto kern_b = kept ? residual_norm_kernel<bf16, true> : residual_norm_kernel<bf16, false>;
+  auto kern_f = kept ? residual_norm_kernel<float, true> : residual_norm_kernel<float, false>;
   int32_t st = allow_max_smem(ctx, compute == KANSO_COMPUTE_BF16 ? (const void*)kern_b
                                                                  : (const void*)kern_f);
   if (st) return st;

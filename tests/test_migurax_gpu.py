@@ -118,7 +118,7 @@ def test_experts(ctx, torch_cuda, compute, experts, top, width, ff):
             assert rel_err(unguard(ctx, y), ref) <= (4e-6 if compute == F32 else 1e-2), (T, path)
 
 
-@pytest.mark.parametrize("width", [64, 50, 1000, 2048, 2052])
+@pytest.mark.parametrize("width", [64, 50, 1000, 2048, 2052, 4096, 4098])
 def test_residual_step(ctx, torch_cuda, width):
     torch = torch_cuda
     rng = np.random.Generator(np.random.PCG64(width))
