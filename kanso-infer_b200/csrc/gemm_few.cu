@@ -164,16 +164,19 @@ __device__ __forceinline__ void few_mma_f16(float (&c)[4], const uint32_t (&a)[4
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Sums that start from the bits of 1.5 * 2^23: below 2^22 in magnitude (here 2^19 at most) the result, read
+// BIASED: sums that start from the bits of 1.5 * 2^23: below 2^22 in magnitude (here 2^19 at most) the result, read
 // as a float, is that value plus the sum. A subtraction, exact, takes the place of a conversion, of which
-// an SM does 16 per clock: 32 of the 35 clocks that a product and its roundings took at 100 rows.
+// an SM does 16 per clock: 32 of the 35 clocks that a product and its roundings took at 100 rows. It is one more
+// operation of the pipe that scales and adds, though, and only the forms of 65..112 rows (and of 128 in two
+// strips a warp), whose few warps are bound by latency, gain by it (few_launch_int8).
 constexpr uint32_t FEW_BIAS = 0x4B400000u;
+template <bool BIASED>
 __device__ __forceinline__ void few_mma_i8(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                            uint32_t b1) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%10,%10,%10,%10};"
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(FEW_BIAS));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(BIASED ? FEW_BIAS : 0u));
 }
 template <typename T>
 __device__ __forceinline__ T lds(const uint8_t* p) {
@@ -331,12 +334,16 @@ __device__ __forceinline__ void few_int8_block(float (&acc)[RT][NT][4], const ui
     const uint64_t dxp = f32x2(d2.x, d2.y);
 #pragma unroll
     for (int r = 0; r < RT; ++r) {
+      constexpr bool BIASED = NT >= 6;
       uint32_t s[4];
-      few_mma_i8(s, a[r], b.x, b.y);
+      few_mma_i8<BIASED>(s, a[r], b.x, b.y);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const uint64_t sum =
-            f32x2_add(f32x2(s[2 * j], s[2 * j + 1]), f32x2(FEW_BIAS | 1u << 31, FEW_BIAS | 1u << 31));
+            BIASED ? f32x2_add(f32x2(s[2 * j], s[2 * j + 1]),
+                               f32x2(FEW_BIAS | 1u << 31, FEW_BIAS | 1u << 31))
+                   : f32x2(__float_as_uint((float)(int)s[2 * j]),
+                           __float_as_uint((float)(int)s[2 * j + 1]));
         const uint64_t term = f32x2_mul(f32x2_mul(dw[r][j], dxp), sum);
         acc[r][n][2 * j] = __fadd_rn(acc[r][n][2 * j], __uint_as_float((uint32_t)term));
         acc[r][n][2 * j + 1] =
@@ -552,11 +559,15 @@ static int32_t few_launch_int8(kanso_cuda_ctx* ctx, int nt, const CUtensorMap& m
   }
   // More than 64 rows: 8 or 14 warps with registers enough. 28 warps of 16 rows x 32 kept 70 each and
   // spilled: 14336 x 4096 at 100 rows 66 us, 60 with 14 warps of 16 rows x 56. Two strips of 16 weight rows to
-  // a warp read an activation once for both (61 us for 128 rows, 66 with one); 112 rows are not even strips.
+  // a warp read an activation once for both (61 us for 128 rows, 66 with one); 112 weight rows are not even strips,
+  // and there 28 warps are the faster ones at more than 112 rows (67.4 and 71.1 us).
   constexpr int RT = TILE == 128 ? 2 : 1;
-  return nt == 12   ? few_launch<FEW_Q8_INT8, TILE, RT, 6, 2, 1>(ctx, map, a, grid)
-         : nt == 14 ? few_launch<FEW_Q8_INT8, TILE, RT, 7, 2, 1>(ctx, map, a, grid)
-                    : few_launch<FEW_Q8_INT8, TILE, RT, 8, 2, 1>(ctx, map, a, grid);
+  if (nt == 12) return few_launch<FEW_Q8_INT8, TILE, RT, 6, 2, 1>(ctx, map, a, grid);
+  if (nt == 14) return few_launch<FEW_Q8_INT8, TILE, RT, 7, 2, 1>(ctx, map, a, grid);
+  if constexpr (TILE == 128)
+    return few_launch<FEW_Q8_INT8, TILE, RT, 8, 2, 1>(ctx, map, a, grid);
+  else
+    return few_launch<FEW_Q8_INT8, TILE, 1, 4, 4, 1>(ctx, map, a, grid);
 }
 
 // How an int8 product is shared out: whole rows per CTA (results bit-identical to the CPU's) while the
@@ -626,7 +637,8 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   if (int8) {
     grid = (int)tiles * share.split;
     a.add = share.split > 1;
-    // groups of rows for 1, 2 or 4 warps of a row group (a test per group cost 45 % at 32 rows)
+    // groups of eight rows, shared out to one warp of a row group, two, or (112 weight rows, 16 groups) four
+    // (a test per group cost 45 % at 32 rows)
     nt = M <= 16 ? 2 : M <= 24 ? 3 : M <= 32 ? 4 : M <= 48 ? 6 : M <= 64 ? 8 : M <= 96 ? 12 : M <= 112 ? 14 : 16;
   } else {
     a.add = true;
