@@ -36,6 +36,8 @@
 // products are exact and accumulate in f32. The error of a K = 4096 product is about 1e-4 of
 // the output scale against the 1e-3 bound. The decode step's chain of matmuls keeps the
 // three-product kernel in gemm_tc.cu.
+#include <algorithm>
+
 #include "gemm_tma_kernel.cuh"
 #include "tensor_map.h"
 
@@ -59,8 +61,8 @@ __global__ void __launch_bounds__(256)
   __shared__ __half tile[PACK_ROWS * PACK_PITCH];
   pdl_launch_dependents();
   pdl_wait();  // x (and the readers of the buffer cleared here) belong to earlier kernels
-  const int64_t cta = blockIdx.y * (int64_t)gridDim.x + blockIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * gridDim.y * blockDim.x;
+  const int64_t cta = (blockIdx.z * (int64_t)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const int64_t nthreads = (int64_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x;
   for (int64_t j = cta * blockDim.x + threadIdx.x; j < zero.n; j += nthreads) zero.p[j] = 0.f;
   const int k0 = blockIdx.x * PACK_K, m0 = blockIdx.y * PACK_ROWS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(256)
   const int m = m0 + lane;
   const int first = blockIdx.x * HALVES;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(tile) + lane * PACK_PITCH;
-  for (int j = warp; j < HALVES && first + j < 2 * units_total; j += 8) {
+  for (int j = warp + 8 * blockIdx.z; j < HALVES && first + j < 2 * units_total; j += 8 * gridDim.z) {
     uint32_t o[4] = {};
     if (k0 < K) {
 #pragma unroll
@@ -115,8 +117,10 @@ template <int FMT>
 static int32_t tm_pack(kanso_cuda_ctx* ctx, const float* x, void* bp, int M, int Mt, int K,
                        int units_total, const TmZero& zero) {
   constexpr int UNITS = FMT == TM_FMT_Q8_0 ? PACK_K / 32 * Q8_BYTES / 16 : 2 * (Q4K_BYTES / 16);
-  const dim3 grid((unsigned)((units_total + UNITS - 1) / UNITS),
-                  (unsigned)((Mt + PACK_ROWS - 1) / PACK_ROWS));
+  dim3 grid((unsigned)((units_total + UNITS - 1) / UNITS),
+            (unsigned)((Mt + PACK_ROWS - 1) / PACK_ROWS));
+  // few tiles: up to four CTAs read one and write a part each (2048 x 1024 at 65 rows, 15 tiles: 10.8 -> 9.9 us)
+  grid.z = (unsigned)std::max<int64_t>(1, std::min<int64_t>(4, ctx->sm_count / ((int64_t)grid.x * grid.y)));
   auto kern = aligned16(x) ? tm_pack_kernel<FMT, true> : tm_pack_kernel<FMT, false>;
   const cudaError_t le = launch_dependent(ctx, kern, grid, dim3(256), 0, x,
                                           reinterpret_cast<__half*>(bp), M, Mt, K, units_total,
@@ -201,8 +205,14 @@ int32_t tma_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   a.ksplit = ksplit;
   a.ub = ub;
   a.status = ctx->dev_status;
-  const size_t smem = (size_t)TM_RAW_SLOTS * TM_BOX + (size_t)TM_A_STAGES * TM_A_STAGE +
+  size_t smem = (size_t)TM_RAW_SLOTS * TM_BOX + (size_t)TM_A_STAGES * TM_A_STAGE +
                       (size_t)b_slots * ub * 32 * Mt + 256;
+  // An SM's shared memory is split in steps, of which 196 KB and 228 KB come into question. A product that leaves no
+  // room for a pack's CTA (16 KB) in the 196 KB asks for a little more than those: else the next pack waits until
+  // the SM has drained and changed its split (18944 x 3584 Q8_0 at 112 rows, 184 KB: 36.9 us, 31.0 with more; at 96
+  // rows, 176 KB, 30.5).
+  constexpr size_t STEP = 196 * 1024, PACK = PACK_ROWS * PACK_PITCH * 2 + 2048;
+  if (smem + 1024 <= STEP && smem + 1024 + PACK > STEP) smem = STEP;
   if (smem > (size_t)ctx->smem_optin)
     return fail(ctx, KANSO_ERR_UNSUPPORTED, "gemm_tma: %zu bytes of shared memory needed", smem);
   const dim3 grid(tiles_n, ksplit);
