@@ -473,7 +473,20 @@ int32_t launch_gemm_pair(kanso_cuda_ctx* ctx, const DenseMat& w, const DenseMat*
   }
   if (most > (1 << 30)) return KANSO_OK;
   t.most = (int)most;
+  // Where the lines lie (us of one product, gemm_dense.cu's form / this one). Rows: below 96 a tile is mostly its
+  // 4 KB of weights per 16 columns, and 32768 x 2048 takes 30.5 / 33.0 at 64 rows, 34.8 / 35.8 at 90, 37.4 / 37.5 at
+  // 128, 60 / 38 at 144; smaller matrices are ahead from 72 rows on. Pairs: with fewer than three quarters of them busy
+  // the other form is the one that can share out the columns too (3072 x 2048 at eight rows 6 in four parts, 11 in
+  // one); in one part pairs are ahead well below that (1024 x 2048 at 256 rows, 4 tiles, 15.9 / 13.2), which
+  // makes this a cautious line.
   if (total * 4 < pairs * 3) return KANSO_OK;
+  // Where all of the other form's tiles lie on the GPU at once, two to an SM, they are ahead if pairs need a second
+  // round (6152 x 2048 at 640 rows 21.7 / 23.9, at 800, which are two rounds either way, 32.6 / 24.8) or have one
+  // tile of the largest size and few columns, where it is stored with nothing behind it to multiply (4096 x 512 at 1024
+  // rows 11.5 / 12.5, 8192 x 1024 at 512 14.9 / 15.3, 2048 x 2048 at 2048 21.1 / 19.9).
+  if (!r.offsets && (w.rows + 127) / 128 * r.groups * ((per + 127) / 128) <= 2 * (int64_t)ctx->sm_count &&
+      (total > pairs || (t.n == GP_MAX_N && w.cols <= 1024)))
+    return KANSO_OK;
   CUtensorMap wm, um, xm;
   int32_t st = weight_map(ctx, w, &wm, up ? 64 : 128);
   if (!st && up) st = weight_map(ctx, *up, &um, 64);
