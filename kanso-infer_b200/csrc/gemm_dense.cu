@@ -1,14 +1,14 @@
 // Tile products of unquantised weights with many activation rows: prompts, batched decoding and
 // the routed experts (grouped rows).
 //
-// bfloat16: a CTA computes 128 weight rows x NT activation rows (two weight tiles of 128 when
-// DUAL), both operands K-major in the 128-byte swizzle, brought by tensor-map copies into a ring
+// bfloat16: a CTA computes 128 weight rows x NT activation rows, both operands K-major in the 128-byte swizzle, brought by tensor-map copies into a ring
 // of shared-memory stages of 64 columns; one thread issues the copies, one the tcgen05.mma
 // (kind::f16, M = 128, N = NT), accumulators in TMEM. The weights take the M side, so that a few
 // activation rows need no padding to 128, and an epilogue warp writes 32 consecutive results of
-// one activation row. DUAL either doubles the weight rows of a CTA or, for the experts, holds the
-// gate and the up accumulator of the same row in the same TMEM lane, so that silu(gate) * up is
-// formed in the epilogue.
+// one activation row. ACT: for the experts, the gate and the up accumulator of the same row lie in the
+// same TMEM lane, so that silu(gate) * up is formed in the epilogue. (Two weight tiles a CTA for plain products too
+// were worth it for large ones, which are gemm_pair.cu's now; of what was left to them, 65 to 95 rows of many
+// weight rows, one tile is the faster: 151936 x 2048 at 80 rows 138 us with two, 127 with one.)
 //
 // Grouped rows: the activation rows are sorted by group (expert); the grid covers the most tiles
 // there can be and a CTA finds its (group, tile) from the offsets on the device, so the host
@@ -71,50 +71,45 @@ __device__ __forceinline__ bool find_tile(const uint32_t* offsets, int groups, i
   return false;
 }
 
-template <int NT, bool DUAL, bool ACT>
+template <int NT, bool ACT>
 struct GdShape {
-  static constexpr int kStage = GD_A_BYTES * (DUAL ? 2 : 1) + NT * 128;
-  // two CTAs per SM for the single form, one for the dual form
-  static constexpr int kStages = DUAL ? (NT <= 32 ? 5 : 4) : NT <= 32 ? 5 : NT <= 64 ? 4 : 3;
-  static constexpr int kCols = (DUAL ? 2 : 1) * NT;
+  static constexpr int kStage = GD_A_BYTES * (ACT ? 2 : 1) + NT * 128;
+  // two CTAs per SM for plain products, one for the experts' two
+  static constexpr int kStages = ACT ? (NT <= 32 ? 5 : 4) : NT <= 32 ? 5 : NT <= 64 ? 4 : 3;
+  static constexpr int kCols = (ACT ? 2 : 1) * NT;
   static constexpr size_t kSmem = (size_t)kStage * kStages + 1024;
 };
 
-// The results of column n (and n + 128) through bias and activation to their places.
-template <int NT, bool DUAL, typename O>
+// The results of column n through bias and activation to their places.
+template <int NT, typename O>
 __device__ __forceinline__ void ext_rows(const GemmDenseArgs& a, const RowPlace& place, O* out,
                                          uint32_t tmem, int n, int64_t first, int valid) {
-  const float b0 = a.bias_of(n), b1 = DUAL ? a.bias_of(n + 128) : 0.f;
-  const bool in0 = n < a.n_end, in1 = DUAL && n + 128 < a.n_end, sq = a.relu2;
+  const float bias = a.bias_of(n);
+  const bool in = n < a.n_end, sq = a.relu2;
   const int64_t ld = a.out_ld;
   out += place.shift + n;
   for (int c = 0; c < NT; c += 16) {
     if (c >= valid) break;
-    uint32_t r0[16], r1[16];
-    tmem_ld16(tmem + c, r0);
-    if (DUAL) tmem_ld16(tmem + NT + c, r1);
+    uint32_t r[16];
+    tmem_ld16(tmem + c, r);
     O* o = out + (first + c) * ld;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       if (c + j >= valid) continue;
-      const float x = __uint_as_float(r0[j]) + b0;
+      const float x = __uint_as_float(r[j]) + bias;
       O* at = place.list ? out + place.list[first + c + j - place.first] * ld : o + j * ld;
-      if (in0) at[0] = to_elem<O>(sq ? relu_squared(x) : x);
-      if (DUAL) {
-        const float y = __uint_as_float(r1[j]) + b1;
-        if (in1) at[128] = to_elem<O>(sq ? relu_squared(y) : y);
-      }
+      if (in) at[0] = to_elem<O>(sq ? relu_squared(x) : x);
     }
   }
 }
 
 // EXT: results go through bias, activation, element type or place (GemmOut).
-template <int NT, bool DUAL, bool ACT, bool EXT>
+template <int NT, bool ACT, bool EXT>
 __global__ void __launch_bounds__(GD_THREADS)
     gemm_dense_kernel(const __grid_constant__ CUtensorMap wmap,
                       const __grid_constant__ CUtensorMap wmap2,
                       const __grid_constant__ CUtensorMap xmap, const GemmDenseArgs a) {
-  using S = GdShape<NT, DUAL, ACT>;
+  using S = GdShape<NT, ACT>;
   extern __shared__ uint8_t raw[];
   __shared__ uint64_t full[S::kStages], empty[S::kStages], acc_full;
   __shared__ uint32_t tmem_slot;
@@ -153,7 +148,7 @@ __global__ void __launch_bounds__(GD_THREADS)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const int n0 = blockIdx.x * 128 * (DUAL && !ACT ? 2 : 1);
+  const int n0 = blockIdx.x * 128;
   const int k0 = blockIdx.z * a.steps_per_split;
   const int k1 = min(k0 + a.steps_per_split, a.k_steps);
 
@@ -169,10 +164,8 @@ __global__ void __launch_bounds__(GD_THREADS)
         uint8_t* st = ring + s * S::kStage;
         mbar_arrive_expect_tx(&full[s], S::kStage);
         tma_load_3d(st, &wmap, k * GD_K, n0, tile_group, &full[s]);
-        if (DUAL)
-          tma_load_3d(st + GD_A_BYTES, ACT ? &wmap2 : &wmap, k * GD_K, ACT ? n0 : n0 + 128,
-                      tile_group, &full[s]);
-        tma_load_2d(st + GD_A_BYTES * (DUAL ? 2 : 1), &xmap, k * GD_K, (int)tile_first, &full[s]);
+        if (ACT) tma_load_3d(st + GD_A_BYTES, &wmap2, k * GD_K, n0, tile_group, &full[s]);
+        tma_load_2d(st + GD_A_BYTES * (ACT ? 2 : 1), &xmap, k * GD_K, (int)tile_first, &full[s]);
         issued = i + 1;
       }
       // leave only when every copy this thread started has landed (bounded)
@@ -195,12 +188,12 @@ __global__ void __launch_bounds__(GD_THREADS)
         const uint32_t base = smem_u32(ring + s * S::kStage);
         const uint64_t ad = tc_smem_desc_sw128(base);
         const uint64_t ad2 = tc_smem_desc_sw128(base + GD_A_BYTES);
-        const uint64_t bd = tc_smem_desc_sw128(base + GD_A_BYTES * (DUAL ? 2 : 1));
+        const uint64_t bd = tc_smem_desc_sw128(base + GD_A_BYTES * (ACT ? 2 : 1));
 #pragma unroll
         for (int j = 0; j < GD_K / 16; ++j) {
           const uint32_t acc = (i > 0 || j > 0) ? 1u : 0u;
           tc_mma_f16(tmem, ad + 2 * j, bd + 2 * j, idesc, acc);
-          if (DUAL) tc_mma_f16(tmem + NT, ad2 + 2 * j, bd + 2 * j, idesc, acc);
+          if (ACT) tc_mma_f16(tmem + NT, ad2 + 2 * j, bd + 2 * j, idesc, acc);
         }
         tc_commit(&empty[s]);
       }
@@ -223,16 +216,16 @@ __global__ void __launch_bounds__(GD_THREADS)
     if (EXT) {
       const RowPlace place(a, tile_group);
       if (a.elem)
-        ext_rows<NT, DUAL>(a, place, static_cast<bf16*>(a.out), lane_base, n, tile_first, valid);
+        ext_rows<NT>(a, place, static_cast<bf16*>(a.out), lane_base, n, tile_first, valid);
       else
-        ext_rows<NT, DUAL>(a, place, static_cast<float*>(a.out) + (int64_t)blockIdx.z * a.part_stride,
-                           lane_base, n, tile_first, valid);
+        ext_rows<NT>(a, place, static_cast<float*>(a.out) + (int64_t)blockIdx.z * a.part_stride,
+                     lane_base, n, tile_first, valid);
     }
     for (int c = 0; c < NT / 16 && !EXT; ++c) {
       if (c * 16 >= valid) break;
       uint32_t r0[16], r1[16];
       tmem_ld16(lane_base + c * 16, r0);
-      if (DUAL) tmem_ld16(lane_base + NT + c * 16, r1);
+      if (ACT) tmem_ld16(lane_base + NT + c * 16, r1);
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int m = c * 16 + j;
@@ -247,7 +240,6 @@ __global__ void __launch_bounds__(GD_THREADS)
           float* o = static_cast<float*>(a.out) + (int64_t)blockIdx.z * a.part_stride +
                      row * a.out_ld;
           if (n < a.rows) o[n] = __uint_as_float(r0[j]);
-          if (DUAL && n + 128 < a.rows) o[n + 128] = __uint_as_float(r1[j]);
         }
       }
     }
@@ -342,14 +334,14 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <int NT, bool DUAL, bool ACT, bool EXT>
+template <int NT, bool ACT, bool EXT>
 static int32_t gd_launch(kanso_cuda_ctx* ctx, dim3 grid, const CUtensorMap& wm,
                          const CUtensorMap& wm2, const CUtensorMap& xm, const GemmDenseArgs& a) {
-  auto kern = gemm_dense_kernel<NT, DUAL, ACT, EXT>;
+  auto kern = gemm_dense_kernel<NT, ACT, EXT>;
   int32_t st = allow_max_smem(ctx, (const void*)kern);
   if (st) return st;
   const cudaError_t e = launch_dependent(ctx, kern, grid, dim3(GD_THREADS),
-                                         GdShape<NT, DUAL, ACT>::kSmem, wm, wm2, xm, a);
+                                         GdShape<NT, ACT>::kSmem, wm, wm2, xm, a);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "gemm_dense launch");
   return after_launch(ctx, "gemm_dense");
 }
@@ -393,9 +385,6 @@ int32_t launch_gemm(kanso_cuda_ctx* ctx, int32_t compute, const DenseMat& w, con
   if (st) return st;
   const int64_t ty = tiles_of(r, nt), tx = (w.rows + 127) / 128;
   a.k_steps = (int)((w.cols + GD_K - 1) / GD_K);
-  // short products spend more time on their ends than the second tile saves: there two CTAs per
-  // SM, of which one stores while the other multiplies
-  const bool dual = nt == 128 && tx * ty >= 4 * (int64_t)ctx->sm_count && a.k_steps >= 12;
   // a share of the columns per CTA while the grid stays within one wave of two CTAs per SM
   int sp = 1;
   while (sp * 2 <= max_splits && tx * ty * sp * 2 <= 2 * (int64_t)ctx->sm_count &&
@@ -404,22 +393,18 @@ int32_t launch_gemm(kanso_cuda_ctx* ctx, int32_t compute, const DenseMat& w, con
   a.steps_per_split = (a.k_steps + sp - 1) / sp;
   sp = (a.k_steps + a.steps_per_split - 1) / a.steps_per_split;
   *splits = sp;
-  auto launch = [&](auto n, auto two, dim3 grid) {
+  const dim3 grid((unsigned)tx, (unsigned)ty, (unsigned)sp);
+  auto launch = [&](auto n) {
     constexpr int NT = decltype(n)::value;
-    constexpr bool DUAL = decltype(two)::value;
-    return ext ? gd_launch<NT, DUAL, false, true>(ctx, grid, wm, wm, xm, a)
-               : gd_launch<NT, DUAL, false, false>(ctx, grid, wm, wm, xm, a);
+    return ext ? gd_launch<NT, false, true>(ctx, grid, wm, wm, xm, a)
+               : gd_launch<NT, false, false>(ctx, grid, wm, wm, xm, a);
   };
   using std::integral_constant;
-  if (dual)
-    return launch(integral_constant<int, 128>(), std::true_type(),
-                  dim3((unsigned)((w.rows + 255) / 256), (unsigned)ty, (unsigned)sp));
-  const dim3 grid((unsigned)tx, (unsigned)ty, (unsigned)sp);
   switch (nt) {
-    case 16: return launch(integral_constant<int, 16>(), std::false_type(), grid);
-    case 32: return launch(integral_constant<int, 32>(), std::false_type(), grid);
-    case 64: return launch(integral_constant<int, 64>(), std::false_type(), grid);
-    default: return launch(integral_constant<int, 128>(), std::false_type(), grid);
+    case 16: return launch(integral_constant<int, 16>());
+    case 32: return launch(integral_constant<int, 32>());
+    case 64: return launch(integral_constant<int, 64>());
+    default: return launch(integral_constant<int, 128>());
   }
 }
 
@@ -449,10 +434,10 @@ int32_t launch_gemm_gate_up(kanso_cuda_ctx* ctx, int32_t compute, const DenseMat
   a.k_steps = a.steps_per_split = (int)((gate.cols + GD_K - 1) / GD_K);
   const dim3 grid((unsigned)((gate.rows + 127) / 128), (unsigned)tiles_of(r, nt));
   switch (nt) {
-    case 16: return gd_launch<16, true, true, false>(ctx, grid, gm, um, xm, a);
-    case 32: return gd_launch<32, true, true, false>(ctx, grid, gm, um, xm, a);
-    case 64: return gd_launch<64, true, true, false>(ctx, grid, gm, um, xm, a);
-    default: return gd_launch<128, true, true, false>(ctx, grid, gm, um, xm, a);
+    case 16: return gd_launch<16, true, false>(ctx, grid, gm, um, xm, a);
+    case 32: return gd_launch<32, true, false>(ctx, grid, gm, um, xm, a);
+    case 64: return gd_launch<64, true, false>(ctx, grid, gm, um, xm, a);
+    default: return gd_launch<128, true, false>(ctx, grid, gm, um, xm, a);
   }
 }
 
