@@ -431,8 +431,10 @@ __global__ void expert_sum_kernel(const float* __restrict__ ye, const uint32_t* 
 
 // Router and choice, one CTA per RW rows: its warps share out the experts, two at a time
 // (logits = router . x + bias in f32), then one warp per row makes the choice (warp_route).
-template <int RW>
-__global__ void __launch_bounds__(DR_THREADS, RW == 1 ? 1 : 4)
+// AHEAD: columns of two experts' weights that are asked for together, AHEAD x 128, the first of them before the
+// wait; CTAS of them an SM (launch_route).
+template <int RW, int AHEAD, int CTAS>
+__global__ void __launch_bounds__(DR_THREADS, CTAS)
     route_kernel(const float* __restrict__ x, int width, const float* __restrict__ router, int ld,
                  const float* __restrict__ bias, int experts, int top, RouteWeights form, uint32_t* __restrict__ sel, float* __restrict__ weight,
                  uint32_t* __restrict__ counts, uint32_t* __restrict__ slot, int64_t T) {
@@ -441,9 +443,6 @@ __global__ void __launch_bounds__(DR_THREADS, RW == 1 ? 1 : 4)
   const int64_t t0 = (int64_t)blockIdx.x * RW;
   float* xw = sm;             // [RW][ld]
   float* l = xw + RW * ld;    // [RW][experts]
-  // Columns of two experts' weights, AHEAD x 128 at a time; the first of them before the wait. One row per
-  // CTA is all latency and takes what 2048 columns have in one go.
-  constexpr int AHEAD = RW == 1 ? 16 : 4;
   float4 a[AHEAD], b[AHEAD];
   auto fetch = [&](int e0, int c0) {
     const float* w0 = router + (int64_t)e0 * ld + c0 + lane * 4;
@@ -889,7 +888,15 @@ int32_t launch_route(kanso_cuda_ctx* ctx, const float* x, int64_t width, const D
   if (smem > 220 * 1024)
     return fail(ctx, KANSO_ERR_UNSUPPORTED, "router: %d experts, width %lld", experts,
                 (long long)width);
-  auto kern = rw == 4 ? route_kernel<4> : route_kernel<1>;
+  // One row a CTA: a row that has an SM to itself is all latency and takes what 2048 columns have in one go (167
+  // registers a thread); more rows than SMs want their CTAs side by side. us, 16 experts of 2048 columns, with one CTA an
+  // SM | with four, five and eight: 300 rows 15.5 | 8.6, 9.5, 10.0; 600 rows 25.1 | 14.7, 10.6, 11.9; 1000 rows
+  // 35.9 | 17.1, 19.9, 15.3.
+  auto kern = rw == 4                  ? route_kernel<4, 4, 4>
+              : T <= ctx->sm_count     ? route_kernel<1, 16, 1>
+              : T <= 4 * ctx->sm_count ? route_kernel<1, 4, 4>
+              : T <= 5 * ctx->sm_count ? route_kernel<1, 2, 5>
+                                       : route_kernel<1, 2, 8>;
   int32_t st = allow_max_smem(ctx, (const void*)kern);
   if (st) return st;
   DR_LAUNCH(kern, (T + rw - 1) / rw, DR_THREADS, smem, "route", x, (int)width,
