@@ -10,6 +10,8 @@
 namespace kanso {
 
 constexpr int DR_THREADS = 256;
+// Wider rows keep the loops through shared memory: two float4 a thread (q and k norm: three) is as far as
+// it was measured, not where it ends to pay.
 constexpr int DR_KEEP = 2;  // float4 of a row that a thread keeps
 
 __device__ __forceinline__ void add4(float4& a, const float4& b) {

@@ -601,10 +601,9 @@ int32_t few_matmul(kanso_cuda_ctx* ctx, int32_t dtype, const void* w, const floa
   const int64_t row_bytes = K / FEW_K * (q4 ? Q4K_BYTES : FEW_K / 32 * Q8_BYTES);
   const int64_t chunks = K / FEW_K;
   // The int8 form is bound by the arithmetic of the SMs that have any: tiles of 112 rows where they
-  // shorten the longest chain of rows on an SM. us at 128 activation rows with 112 and with 128 when a
-  // warp still had 32 of them: 14336 x 4096 (128 and 112 busy SMs) 100 and 106 with cold caches; 17408 x
-  // 4096, two waves of 112 rows and one of 128, 130 and 72 behind one another, 18944 x 3584 115 and 64.
-  // With 56 rows a warp (14336 x 4096, 100 rows): 60.0 and 60.5.
+  // shorten the longest chain of rows on an SM. us at 100 and 128 activation rows with 112 | with 128: 14336 x 4096
+  // (128 and 112 busy SMs) 62, 68 | 63, 71; 10500 x 4096 62, 68 | 66, 75; 17408 x 4096 (two waves of 112 rows,
+  // one of 128) 118, 131 | 63, 72; 18944 x 3584 104, 116 | 56, 64.
   const FewShare s128 = few_share(ctx, 128, N, chunks), s112 = few_share(ctx, 112, N, chunks);
   const FewShare& share = int8 && s112.chain < s128.chain ? s112 : s128;
   const int tile = share.tile;

@@ -25,8 +25,8 @@ constexpr int TM_A_STAGES = 2;
 constexpr int TM_A_STAGE = 32768;  // 16 k-chunks of 8 positions x 128 rows x 16 bytes
 // Activation ring: four slots of up to 16 KB for the two issuing threads of up to 128 rows, three of up
 // to 32 KB for the one of more rows. That thread pays about 500 cycles a slot for the wait, the fence and
-// the commit, whatever the slot holds: 512 rows of 14336 x 4096 in slots of one k-step 79 us, of
-// two 71 us; 256 rows in slots of two and of four 47 and 41 us.
+// the commit, whatever the slot holds: product and pack of 512 rows of 14336 x 4096 79 us in slots of one k-step,
+// 71 of two; 256 rows in slots of two and of four 47 and 41.
 constexpr int TM_B_SLOTS_TWO = 4, TM_B_SLOT_TWO = 16384;
 constexpr int TM_B_SLOTS_ONE = 3, TM_B_SLOT_ONE = 32768;
 constexpr int TM_B_SLOTS_MAX = 4;
@@ -291,9 +291,9 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
   // odd stages), because a tcgen05.mma of few columns is bound by the issuing thread, not by the
   // tensor core (measured: 8 MMAs + commit cost one thread 873 cycles at N = 32 whether or not a
   // second thread issues beside it). The epilogue adds the two accumulators. With more rows a
-  // stage takes all four activation slots, so both threads would use every slot in turn and the
-  // second would have to wait for a slot's second filling without having seen its first (a
-  // parity wait cannot express that); those sizes are bound by the tensor core anyway.
+  // stage takes two or four fillings of the ring's three activation slots, so both threads would use every
+  // slot in turn and the second would have to wait for a slot's second filling without having seen its first
+  // (a parity wait cannot express that); those sizes are bound by the tensor core anyway.
   const int nissue = a.Mt <= 128 ? 2 : 1;
   uint32_t acc_cols = 32;
   while (acc_cols < (uint32_t)a.Mt) acc_cols <<= 1;

@@ -262,6 +262,8 @@ __device__ __forceinline__ bool gate_source_wide(const GemvSource& s, int cols, 
 // registers. Every CTA of a product forms its input, so that its latency is the product's: with one row, one
 // float and one pass after another 4096 x 2048 behind a residual step took 19.3 us at two rows, 12.2 so, and 9.4
 // once every CTA stays for the whole product (gv_grid).
+// Wider rows, and gated ones beyond 2048 columns or with heads that are no multiple of 128, keep the loops below: two
+// float4 a thread is as far as it was measured, not where it ends to pay.
 constexpr int GV_KEEP = 2;  // float4 of a row that a thread keeps
 template <int TT, int KIND>
 __device__ __forceinline__ bool norm_source_wide(const GemvSource& s, int cols, int ld, int t0, int nt,

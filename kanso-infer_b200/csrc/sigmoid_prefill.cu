@@ -17,7 +17,7 @@
 // tab[d] = -log2(e) * (cap + pb - r1 ln(1 + r2 d)) for visible distances and +infinity for the
 // others, so that a masked weight is 1 / (1 + 2^inf) = 0 without a comparison.
 //
-// us at 2048 rows behind 2048 cached ones, 16 heads of 128, window 1024: 137 with one copying warp, a ring
+// us at 2048 rows behind 2048 cached ones, 16 heads of 128, window 2048: 137 with one copying warp, a ring
 // of two and one issuing thread, where every tile took a copy's round trip; 98 with warps and rings of their own and reciprocals shared, 85 with three groups.
 #include <algorithm>
 

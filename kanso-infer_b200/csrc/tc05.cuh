@@ -8,6 +8,12 @@
 namespace kanso {
 
 // ---- tcgen05 wrappers ----
+// A CTA that asks for columns which another one on its SM holds waits without a limit, so that none may hold
+// columns across griddepcontrol.wait while a CTA of a kernel in front still wants some there. gemm_tc_kernel and
+// gemm_tma_kernel take theirs in front of that wait all the same: with 148 and 144 KB of shared memory at the
+// least they share an SM with none of the others that take columns (gemm_dense_kernel 91 KB and more,
+// softmax_prefill_kernel 113, sigmoid_prefill_kernel 130, gemm_pair_kernel 193, of an SM's 228). Whoever takes less
+// takes its columns behind the wait.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                    smem_u32(dst_smem)),

@@ -61,7 +61,7 @@ def test_linear_with_bias_and_squared_relu(ctx, torch_cuda, compute, rows, cols)
 
 @pytest.mark.parametrize("compute, path, T, rows", [
     (F32, 1, 2, 50), (F32, 2, 40, 50), (BF16, 1, 2, 50), (BF16, 2, 40, 300),
-    (BF16, 2, 70, 80000),   # two tiles of weight rows for each CTA
+    (BF16, 2, 70, 80000),   # more tiles than the GPU holds at once
     (BF16, 2, 100, 14400),  # pairs of CTAs
 ])
 def test_linear_keeps_what_is_no_number(ctx, torch_cuda, compute, path, T, rows):
