@@ -136,10 +136,17 @@ __global__ void __launch_bounds__(256)
                       silu_mul_one(a[j].z, b[j].z), silu_mul_one(a[j].w, b[j].w));
     return;
   }
+  float a[SILU_PER], b[SILU_PER];  // all loads in front of the stores: out may be where g or u is
 #pragma unroll
   for (int j = 0; j < SILU_PER; ++j) {
     const int64_t i = base + j * 256 + threadIdx.x;
-    if (i < n) out[i] = silu_mul_one(g[i], u[i]);
+    a[j] = i < n ? g[i] : 0.f;
+    b[j] = i < n ? u[i] : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < SILU_PER; ++j) {
+    const int64_t i = base + j * 256 + threadIdx.x;
+    if (i < n) out[i] = silu_mul_one(a[j], b[j]);
   }
 }
 
@@ -165,10 +172,17 @@ __global__ void __launch_bounds__(256) residual_add_kernel(float* h, const float
           make_float4(a[j].x + b[j].x, a[j].y + b[j].y, a[j].z + b[j].z, a[j].w + b[j].w);
     return;
   }
+  float a[SILU_PER], b[SILU_PER];  // all loads in front of the stores, which may be to where others come from
 #pragma unroll
   for (int j = 0; j < SILU_PER; ++j) {
     const int64_t i = base + j * 256 + threadIdx.x;
-    if (i < n) h[i] = h[i] + p[i];
+    a[j] = i < n ? h[i] : 0.f;
+    b[j] = i < n ? p[i] : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < SILU_PER; ++j) {
+    const int64_t i = base + j * 256 + threadIdx.x;
+    if (i < n) h[i] = a[j] + b[j];
   }
 }
 
