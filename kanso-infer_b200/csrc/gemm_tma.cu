@@ -36,8 +36,6 @@
 // products are exact and accumulate in f32. The error of a K = 4096 product is about 1e-4 of
 // the output scale against the 1e-3 bound. The decode step's chain of matmuls keeps the
 // three-product kernel in gemm_tc.cu.
-#include <algorithm>
-
 #include "gemm_tma_kernel.cuh"
 #include "tensor_map.h"
 
@@ -51,7 +49,8 @@ namespace kanso {
 // Tiles behind the last k are the stream's padding: zeros.
 constexpr int PACK_ROWS = 32, PACK_K = 256;
 constexpr int PACK_PITCH = PACK_K + 2;  // an odd number of words: lanes along the rows, 32 banks
-template <int FMT, bool VEC>
+// PARTS: CTAs that read one tile and write a part of it each (blockIdx.z).
+template <int FMT, bool VEC, int PARTS>
 __global__ void __launch_bounds__(256)
     tm_pack_kernel(const float* __restrict__ x, __half* __restrict__ bp, int M, int Mt, int K,
                    int units_total, const TmZero zero) {
@@ -97,7 +96,7 @@ __global__ void __launch_bounds__(256)
   const int m = m0 + lane;
   const int first = blockIdx.x * HALVES;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(tile) + lane * PACK_PITCH;
-  for (int j = warp + 8 * blockIdx.z; j < HALVES && first + j < 2 * units_total; j += 8 * gridDim.z) {
+  for (int j = warp + 8 * blockIdx.z; j < HALVES && first + j < 2 * units_total; j += 8 * PARTS) {
     uint32_t o[4] = {};
     if (k0 < K) {
 #pragma unroll
@@ -119,9 +118,13 @@ static int32_t tm_pack(kanso_cuda_ctx* ctx, const float* x, void* bp, int M, int
   constexpr int UNITS = FMT == TM_FMT_Q8_0 ? PACK_K / 32 * Q8_BYTES / 16 : 2 * (Q4K_BYTES / 16);
   dim3 grid((unsigned)((units_total + UNITS - 1) / UNITS),
             (unsigned)((Mt + PACK_ROWS - 1) / PACK_ROWS));
-  // few tiles: up to four CTAs read one and write a part each (2048 x 1024 at 65 rows, 15 tiles: 10.8 -> 9.9 us)
-  grid.z = (unsigned)std::max<int64_t>(1, std::min<int64_t>(4, ctx->sm_count / ((int64_t)grid.x * grid.y)));
-  auto kern = aligned16(x) ? tm_pack_kernel<FMT, true> : tm_pack_kernel<FMT, false>;
+  // few tiles: two or four CTAs share one (2048 x 1024 at 65 rows, 15 tiles: 10.8 -> 9.9 us)
+  const int64_t room = ctx->sm_count / ((int64_t)grid.x * grid.y);
+  grid.z = room >= 4 ? 4 : room >= 2 ? 2 : 1;
+  const bool vec = aligned16(x);
+  auto kern = grid.z == 4   ? (vec ? tm_pack_kernel<FMT, true, 4> : tm_pack_kernel<FMT, false, 4>)
+              : grid.z == 2 ? (vec ? tm_pack_kernel<FMT, true, 2> : tm_pack_kernel<FMT, false, 2>)
+                            : (vec ? tm_pack_kernel<FMT, true, 1> : tm_pack_kernel<FMT, false, 1>);
   const cudaError_t le = launch_dependent(ctx, kern, grid, dim3(256), 0, x,
                                           reinterpret_cast<__half*>(bp), M, Mt, K, units_total,
                                           zero);
