@@ -560,14 +560,16 @@ static int32_t few_launch_int8(kanso_cuda_ctx* ctx, int nt, const CUtensorMap& m
   // More than 64 rows: 8 or 14 warps with registers enough. 28 warps of 16 rows x 32 kept 70 each and
   // spilled: 14336 x 4096 at 100 rows 66 us, 60 with 14 warps of 16 rows x 56. Two strips of 16 weight rows to
   // a warp read an activation once for both (61 us for 128 rows, 66 with one); 112 weight rows are not even strips,
-  // and there 28 warps are the faster ones at more than 112 rows (67.4 and 71.1 us).
+  // and there 28 warps are the faster ones at more than 112 rows (68.1 and 70.7 us; 4096 x 14336 63.4 and 65.8), but
+  // not where K is split and a CTA has no more than four units (4096 x 2048 16.5 and 16.0, 4096 x 4096 24.4 and 24.3).
   constexpr int RT = TILE == 128 ? 2 : 1;
   if (nt == 12) return few_launch<FEW_Q8_INT8, TILE, RT, 6, 2, 1>(ctx, map, a, grid);
   if (nt == 14) return few_launch<FEW_Q8_INT8, TILE, RT, 7, 2, 1>(ctx, map, a, grid);
-  if constexpr (TILE == 128)
-    return few_launch<FEW_Q8_INT8, TILE, RT, 8, 2, 1>(ctx, map, a, grid);
-  else
-    return few_launch<FEW_Q8_INT8, TILE, 1, 4, 4, 1>(ctx, map, a, grid);
+  if constexpr (TILE == 112) {
+    if (!(a.add && a.units <= 4 * grid))
+      return few_launch<FEW_Q8_INT8, TILE, 1, 4, 4, 1>(ctx, map, a, grid);
+  }
+  return few_launch<FEW_Q8_INT8, TILE, RT, 8, 2, 1>(ctx, map, a, grid);
 }
 
 // How an int8 product is shared out: whole rows per CTA (results bit-identical to the CPU's) while the

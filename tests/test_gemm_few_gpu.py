@@ -149,6 +149,20 @@ def test_q8_activations_halved_k_repeats(ctx, kb, oracle, torch_cuda, M, N, K):
         assert (got[0] == again).all()
 
 
+# K in four and eight parts of two, four and five units a CTA: 14 warps, and 28. The parts' sums are added in
+# any order (1e-5, as above).
+@pytest.mark.parametrize("M", [113, 128])
+@pytest.mark.parametrize("N,K", [(2048, 2048), (2048, 8192), (2048, 10240)])
+def test_q8_activations_in_parts(ctx, kb, oracle, torch_cuda, M, N, K):
+    blocks = matrix("q8_0", N, K)
+    x = data(M, 1, K)[1]
+    got = several_calls(ctx, kb, torch_cuda, "q8_0", blocks, x, N, kb.ACT_Q8)[0]
+    pick = np.r_[0:130, N - 40:N]
+    ref = oracle.gemm_q8_0(np.ascontiguousarray(blocks[pick]).reshape(-1), x, M,
+                           len(pick), K, oracle.ACT_Q8)
+    assert rel_err(got[:, pick], ref) <= 1e-5
+
+
 @pytest.mark.parametrize("M", [513, 530, 576, 584])
 @pytest.mark.parametrize("fmt", ["q8_0", "q4_k"])
 def test_rows_behind_a_pass_of_512(ctx, kb, oracle, torch_cuda, fmt, M):
