@@ -105,8 +105,9 @@ inline cudaError_t launch_dependent(kanso_cuda_ctx* ctx, void (*kern)(KArgs...),
 }
 
 // Launches inside a scope of this kind carry no such attribute: for calls of their own on kernels that read
-// positions, tables and lengths before the wait. A model's step uploads those before its first kernel; a
-// caller of a single mechanism may have them written by the kernel in front.
+// positions and tables, or a state that earlier steps left, before the wait. A model's step uploads the one
+// and starts behind the other's last kernel; a caller of a single mechanism may have them written by a kernel
+// that is still running.
 struct PlainLaunches {
   kanso_cuda_ctx* ctx;
   const bool was;

@@ -189,6 +189,7 @@ int32_t kanso_cuda_mlstm(kanso_cuda_ctx* ctx, kanso_cuda_kv* kv, uint32_t layer,
                          const float* i_bias, const float* f_bias, float* out,
                          const kanso_mlstm_params* p, int32_t path) {
   if (!ctx) return fail(nullptr, KANSO_ERR_CONFIG, "mlstm: ctx is NULL");
+  const PlainLaunches plain(ctx);
   if (!kv || !y || !i_bias || !f_bias || !out || !p)
     return fail(ctx, KANSO_ERR_SHAPE, "mlstm: NULL argument");
   if (!aligned16(y) || !aligned16(out))

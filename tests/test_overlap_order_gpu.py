@@ -13,7 +13,7 @@ import plain_migurax as plain
 import plain_revitar
 from conftest import rel_err
 from revitar_cases import to_bf16
-from test_migurax_gpu import LatentCase, dev, f32, f64, guarded, unguard
+from test_migurax_gpu import LatentCase, Memory, dev, f32, f64, guarded, unguard
 from test_revitar_gpu import BF16, F32, PagedCase, to_dev, u32, unit_rows, up8
 
 pytestmark = pytest.mark.gpu
@@ -250,3 +250,33 @@ def test_router_of_experts(eager, torch_cuda, T, path, which):
              up.data_ptr(), down.data_ptr(), y.data_ptr(), T, width, ff, experts, 2, path)
     ref = plain.moe(f64(x), plain.doubles(w), "", {"router": {"experts": experts, "top": 2}})
     assert rel_err(unguard(ctx, y), ref) <= 4e-6
+
+
+@pytest.mark.parametrize("rows, path", [(1, 1), (20, 1), (130, 2)])
+@pytest.mark.parametrize("which", ["y", "i", "f"])
+def test_matrix_memory(kb, eager, torch_cuda, rows, path, which):
+    """Projections and gate biases written late, from a state that a call before left."""
+    (ctx, late), torch = eager, torch_cuda
+    rng = np.random.Generator(np.random.PCG64(rows))
+    H, D, V, before = 2, 24, 40, 30
+    m = Memory(kb, ctx, torch, H, D, V, 9.0)
+    a = m.inputs(rng, before + rows)
+    ib, fb = f32(rng.standard_normal(H)), f32(rng.standard_normal(H))
+    y = f32(np.concatenate([x.reshape(before + rows, -1) for x in a], axis=1))
+
+    def call(part, pos0, path, is_late):
+        n = part.shape[0]
+        given = {"y": part, "i": ib, "f": fb}
+        arrays = {k: dev(torch, v) for k, v in given.items()}
+        out, p = guarded(torch, n, H * V), kb.MlstmParams(n, pos0, 0, m.cap)
+        if is_late:
+            arrays[which], keep = late(f32(given[which]))
+        ctx.call("kanso_cuda_mlstm", m.pool.h, 0, arrays["y"].data_ptr(), arrays["i"].data_ptr(),
+                 arrays["f"].data_ptr(), out.data_ptr(), ctypes.byref(p), path)
+        return unguard(ctx, out).reshape(n, H, V)
+
+    call(y[:before], 0, 1, False)
+    got = call(y[before:], before, path, True)
+    ref = m.reference(*a[:4], a[4] + ib, a[5] + fb)[before:]
+    assert m.close(got, ref, 1e-4 if path == 1 else 5e-3)
+    m.pool.destroy()
