@@ -167,8 +167,8 @@ __device__ __forceinline__ void few_mma_f16(float (&c)[4], const uint32_t (&a)[4
 // BIASED: sums that start from the bits of 1.5 * 2^23: below 2^22 in magnitude (here 2^19 at most) the result, read
 // as a float, is that value plus the sum. A subtraction, exact, takes the place of a conversion, of which
 // an SM does 16 per clock: 32 of the 35 clocks that a product and its roundings took at 100 rows. It is one more
-// operation of the pipe that scales and adds, though, and only the forms of 65..112 rows (and of 128 in two
-// strips a warp), whose few warps are bound by latency, gain by it (few_launch_int8).
+// operation of the pipe that scales and adds, though, and only the forms of 8 or 14 warps above 64 rows, which are
+// bound by latency, gain by it (few_launch_int8): with it 17 to 64 rows took 3.5 % longer.
 constexpr uint32_t FEW_BIAS = 0x4B400000u;
 template <bool BIASED>
 __device__ __forceinline__ void few_mma_i8(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0,
